@@ -75,16 +75,6 @@ struct SceneCtl {
 // poll is an L2 round trip)
 constexpr long kBarrierSpins = 1L << 26;
 
-// colour-ordered records of the coloured velocity sweeps (layout and packing in pdem_solve.cuh,
-// kPackPgs): kPgsSlots slots of 4 values per entry, slot-major, and the entry's ids
-constexpr int kPgsSlots = 11;
-template <class R>
-struct PgsRecs {
-  Q4<R>* q;
-  int4* ids;
-  long cap;
-};
-
 template <class R>
 struct Dev {
   int cap = 0, maxPairs = 0, maxContacts = 0;

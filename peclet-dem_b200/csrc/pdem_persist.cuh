@@ -75,12 +75,10 @@ __device__ __forceinline__ bool loopBarrier(const GridBar& gb) {
   }
   return gridBarrier(gb);
 }
-// KIND 3: the projected GS velocity sweep of KIND 0 from the colour-ordered records of kPackPgs
-// (entry t of the order is record t), the same arithmetic with fewer dependent loads. The colour
-// offsets (at most 63 colours) are read once into shared memory.
+// The colour offsets (at most 63 colours) are read once into shared memory.
 template <class R, int KIND, int LOOP, bool CLUSTER = false>
 __global__ void __launch_bounds__(kBlock) kSweepLoop(Dev<R> d, const int* order, const int* coff, int ncol, int iters,
-                                                     SolveP<R> P, R thr, GridBar gb, PgsRecs<R> recs) {
+                                                     SolveP<R> P, R thr, GridBar gb) {
   __shared__ int sOff[kSaturatedColor + 2];
   Counters<R>* c = d.ctr;
   volatile int* done = LOOP == 1 ? &c->velDone : LOOP == 2 ? &c->stabDone : &c->posDone;
@@ -106,10 +104,6 @@ __global__ void __launch_bounds__(kBlock) kSweepLoop(Dev<R> d, const int* order,
             pgsOne(d, order[b + t], P, mx, LOOP);
           } else if (KIND == 1) {
             gsOne(d, order[b + t], P, mx);
-          } else if (KIND == 3) {
-            int idx;
-            const PgsStatic<R> st = pgsRecord(recs, b + t, idx);
-            pgsCore<R>(d, idx, st, P.eN, P.mu, 0, P, mx);
           } else {
             posGSOne(d, order[b + t], mx);
           }
@@ -716,6 +710,11 @@ __device__ void colorTailShared(const Dev<R>& d, const ColorJob& jm, const Color
       prevC = remC;
     }
     __syncthreads();  // the counters are read before the next round resets them
+  }
+  for (int s = threadIdx.x; s < kTailShSlots; s += blockDim.x) {  // the bodies' colour masks
+    const int code = S.body[s];
+    if (code >= 0)
+      ((code & 1) ? jc.mask : jm.mask)[code >> 1] = S.mask[s];
   }
 }
 

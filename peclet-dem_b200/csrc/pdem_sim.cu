@@ -10,6 +10,7 @@
 
 #include "pdem_broad.cuh"
 #include "pdem_contact.cuh"
+#include "pdem_flow.cuh"
 #include "pdem_hertz.cuh"
 #include "pdem_kernels.cuh"
 #include "pdem_multilevel.cuh"
@@ -340,22 +341,125 @@ bool Sim<R>::launchClusterCfg(K kernel, int blocks, int block, size_t smem, A...
   return true;
 }
 
-// the colour-ordered velocity-sweep records of this substep's manifolds, packed at the first
-// request of a substep (the orientations and masses they hold do not change until the
-// integration after the stabilization pass)
+// One sweep loop as a flow of body states (pdem_flow.cuh) over the manifolds (KIND 0) or contacts
+// (KIND 2) of the substep. Returns false (nothing launched) where the colour order has the saturated
+// colour, which is not an independent set, where no cluster or grid of it can be resident, and for
+// colours of more entries than the chip takes at once (one group a SM): there a colour step is bound by
+// throughput, the records cost more than they save (262,144 periodic spheres, 240,000 contacts: 21.2 ms
+// per ten substeps by colour, 26.3 ms as a flow; 20,011 spheres in a bed, 61,000: 52.7 against 37.4).
+//
+// Blocks: one thread-block cluster while its shared memory holds every mailbox (about 14,000 velocity
+// entries in double, 32,768 in float), with about kFlowClusterPer entries of a colour a block, so that a
+// small graph's states travel inside few SMs; else one block a SM or fewer, by kFlowGridPer.
+constexpr int kFlowClusterPer = 64, kFlowGridPer = 64;
 template <class R>
-PgsRecs<R> Sim<R>::packPgs(int nm, int ncol) {
-  if (pgsPackedAt_ != substepId_) {
-    // the slot stride is the ids' capacity, so the slots are sized from it after it grew
-    pgsIds_.ensure((size_t)nm, false, stream_);
-    pgsCap_ = (long)(pgsIds_.n);
-    pgsQ_.ensure((size_t)kPgsSlots * pgsIds_.n, false, stream_);
-    ++launches_, kPackPgs<R><<<gridFor(nm), kBlock, 0, stream_>>>(d_, mOrder_.p, mOff_.p, ncol,
-                                                                 PgsRecs<R>{pgsQ_.p, pgsIds_.p, pgsCap_});
-    KCHECK("pack velocity records");
-    pgsPackedAt_ = substepId_;
+template <int KIND, int LOOP>
+bool Sim<R>::flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr) {
+  using F = FlowShape<R, KIND>;
+  const int perColor = (ne + ncol - 1) / ncol;
+  if (ncol > kSaturatedColor || ne >= (1 << 28) || perColor > numSMs_ * kFlowGroup)
+    return false;
+  FlowBuf& f = KIND == 0 ? flowM_ : flowC_;
+  const int* order = KIND == 0 ? mOrder_.p : cOrder_.p;
+  const int* off = KIND == 0 ? mOff_.p : cOff_.p;
+  const u64* mask = KIND == 0 ? mask_.p : maskP_.p;
+  int nb = 1;
+  while (nb < sweepClusterBlocks_ && nb * kFlowClusterPer < perColor)
+    nb *= 2;
+  const int stride = ne / nb + ncol + 1;
+  const size_t smem = F::kStageBytes + (size_t)stride * F::kSlotBytes;
+  auto* kc = kFlowSweeps<R, KIND, LOOP, true>;
+  auto* kg = kFlowSweeps<R, KIND, LOOP, false>;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  cfg.blockDim = dim3(kFlowBlock);
+  cfg.stream = stream_;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const bool fits = ne <= sweepClusterEntries_ && stride < (1 << 14) && smem <= kFlowMaxSmem &&
+                    ne / (nb * kFlowGroup) + ncol < kFlowItems;
+  auto resident = [&](const void* k, int blocks) -> int& { return flowOk_.emplace(std::make_pair(k, blocks), -1).first->second; };
+  bool cluster = fits;
+  if (fits) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nb;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(nb);
+    int& ok = resident(reinterpret_cast<const void*>(kc), nb);
+    if (ok < 0) {  // once per cluster size, with the largest shared memory it may ask for
+      cfg.dynamicSmemBytes = kFlowMaxSmem;
+      int clusters = 0;
+      if (cudaFuncSetAttribute(kc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlowMaxSmem) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&clusters, kc, &cfg) != cudaSuccess)
+        (void)cudaGetLastError();
+      ok = clusters >= 1 ? 1 : 0;
+    }
+    cfg.dynamicSmemBytes = smem;
+    cluster = ok == 1;
   }
-  return PgsRecs<R>{pgsQ_.p, pgsIds_.p, pgsCap_};
+  int grid = 0;
+  if (!cluster) {
+    grid = std::max(1, std::min(numSMs_, (perColor + kFlowGridPer - 1) / kFlowGridPer));
+    if (ne / (grid * kFlowGroup) + ncol >= kFlowItems)
+      return false;
+    int& per = resident(reinterpret_cast<const void*>(kg), 0);
+    if (per < 0) {
+      if (cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, F::kStageBytes) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kg, kFlowBlock, F::kStageBytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        per = 0;
+      }
+    }
+    if (per < 1)
+      return false;
+  }
+  const int target = cluster ? nb : 0;
+  if (f.packedAt != substepId_ || f.blocks != target) {
+    f.rec.ensure((size_t)ne * F::kStride, false, stream_);
+    if (KIND == 0)
+      f.var.ensure((size_t)ne, false, stream_);
+    else
+      f.lam.ensure((size_t)ne, false, stream_);
+    f.tab.ensure((size_t)std::max(KIND == 0 ? numReal_ : numParticles_, 1) * ncol, false, stream_);
+  }
+  FlowRecs<R> rec{f.rec.p, f.var.p, f.lam.p, nullptr, nullptr, 0, 0u};
+  if (f.packedAt != substepId_) {
+    ++launches_, kFlowPack<R, KIND><<<gridFor(ne), kBlock, 0, stream_>>>(d_, order, off, ncol, mask, f.tab.p, rec);
+    KCHECK("flow records");
+    f.blocks = -1;
+  }
+  if (f.blocks != target) {
+    ++launches_, kFlowLink<<<gridFor(ne, kFlowBlock), kFlowBlock, 0, stream_>>>(
+        off, ncol, mask, f.tab.p, KIND == 0 ? mColor_.p : cColor_.p, f.rec.p, F::kStride, F::kIds, target);
+    KCHECK("flow links");
+  }
+  f.packedAt = substepId_;
+  f.blocks = target;
+  const GridBar gb{nullptr, &ctr_.p->err, 0u, barrierSpins_};
+  ++launches_;
+  if (cluster) {
+    cudaCheck(cudaLaunchKernelEx(&cfg, kc, d_, off, ncol, iters, P, thr, gb, rec, stride), "flow sweeps (cluster)");
+  } else {
+    f.box.ensure(2 * (size_t)F::kPackets * ne, false, stream_);
+    rec.cap = (long)(f.box.n / (2 * F::kPackets));
+    f.ctl.ensure(kFlowCtlWords, false, stream_);
+    f.ctl.zero(stream_);
+    if (f.tag > 0xF0000000u) {  // the tags start again
+      f.box.zero(stream_);
+      f.tag = 0;
+    }
+    rec.box = f.box.p;
+    rec.ctl = f.ctl.p;
+    rec.tag0 = f.tag;
+    f.tag += (unsigned)iters + 2u;
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.dynamicSmemBytes = F::kStageBytes;
+    cudaCheck(cudaLaunchKernelEx(&cfg, kg, d_, off, ncol, iters, P, thr, gb, rec, 0), "flow sweeps (grid)");
+  }
+  return true;
 }
 
 // ---- CUB helpers ----
@@ -1611,16 +1715,14 @@ void Sim<R>::demStep() {
       ++launches_, kSweepScenes<R, 0, 1><<<numScenes_, sceneBlock(), 0, s>>>(d_, sceneLpt_.p, mOrder_.p, mOff_.p, velIters_, sp, thr);
     else if (batch_)
       ++launches_, kSweepScenes<R, 1, 1><<<numScenes_, sceneBlock(), 0, s>>>(d_, sceneLpt_.p, mOrder_.p, mOff_.p, velIters_, sp, thr);
-    else if (usePGS && !(nm <= sweepClusterEntries_ &&
-                         launchCluster(kSweepLoop<R, 3, 1, true>, d_, (const int*)mOrder_.p, (const int*)mOff_.p,
-                                       ncolV, velIters_, sp, thr, gb, packPgs(nm, ncolV))))
-      launchCoop(kSweepLoop<R, 0, 1>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, velIters_, sp, thr, gb,
-                 PgsRecs<R>{});
+    else if (usePGS) {
+      if (!flowSweeps<0, 1>(nm, ncolV, velIters_, sp, thr))
+        launchCoop(kSweepLoop<R, 0, 1>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, velIters_, sp, thr, gb);
+    }
     else if (!usePGS && !(nm <= sweepClusterEntries_ &&
                           launchCluster(kSweepLoop<R, 1, 1, true>, d_, (const int*)mOrder_.p, (const int*)mOff_.p,
-                                        ncolV, velIters_, sp, thr, gb, PgsRecs<R>{})))
-      launchCoop(kSweepLoop<R, 1, 1>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, velIters_, sp, thr, gb,
-                 PgsRecs<R>{});
+                                        ncolV, velIters_, sp, thr, gb)))
+      launchCoop(kSweepLoop<R, 1, 1>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, velIters_, sp, thr, gb);
     KCHECK("velocity loop");
   }
   // no colours and no fallback: the first sweep is empty, its END finds maxApproach = 0 <= thr
@@ -1703,7 +1805,11 @@ void Sim<R>::demStep() {
     } else if (stabRun) {
       if (stabMode_ == 1 && nm > 0) {
         ensureGrounded();
-        ++launches_, kSideFlags<<<gridFor(nm), B, 0, s>>>(d_, nm, gHat, R(8) * dt_ * gMag, R(8) * dt_ * gMag);
+        ++launches_, kSideFlags<<<gridFor(nm), B, 0, s>>>(d_, nm, gHat, R(8) * dt_ * gMag, R(8) * dt_ * gMag, mOrder_.p,
+                                                           flowM_.packedAt == substepId_
+                                                               ? flowM_.rec.p + FlowShape<R, 0>::kIds + 3 * sizeof(int)
+                                                               : nullptr,
+                                                           FlowShape<R, 0>::kStride, kFlowSideShift);
       }
       SolveP<R> ss = sp;
       ss.vRest = vRestS;
@@ -1715,11 +1821,8 @@ void Sim<R>::demStep() {
         ctl(CTL_STAB_BEGIN, R(0), 0);
         if (batch_)
           ++launches_, kSweepScenes<R, 0, 2><<<numScenes_, sceneBlock(), 0, s>>>(d_, sceneLpt_.p, mOrder_.p, mOff_.p, iters, ss, vRestS);
-        else if (!(nm <= sweepClusterEntries_ &&
-                   launchCluster(kSweepLoop<R, 3, 2, true>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV,
-                                 iters, ss, vRestS, gb, packPgs(nm, ncolV))))
-          launchCoop(kSweepLoop<R, 0, 2>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, iters, ss, vRestS, gb,
-                     PgsRecs<R>{});
+        else if (!flowSweeps<0, 2>(nm, ncolV, iters, ss, vRestS))
+          launchCoop(kSweepLoop<R, 0, 2>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, iters, ss, vRestS, gb);
       }
       for (int it = 0; it < (stabPersistent ? 0 : iters); ++it) {
         ctl(CTL_STAB_BEGIN, R(0), 0);
@@ -1822,11 +1925,8 @@ void Sim<R>::demStep() {
       ++launches_, kSweepScenes<R, 2, 3><<<numScenes_, sceneBlock(), 0, s>>>(d_, sceneLpt_.p, cOrder_.p, cOff_.p, posIters_, sp, posTol);
       tuneEnd();
     }
-    else if (!(nc <= sweepClusterEntries_ &&
-               launchCluster(kSweepLoop<R, 2, 3, true>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP,
-                             posIters_, sp, posTol, gb, PgsRecs<R>{})))
-      launchCoop(kSweepLoop<R, 2, 3>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP, posIters_, sp, posTol, gb,
-                 PgsRecs<R>{});
+    else if (!flowSweeps<2, 3>(nc, ncolP, posIters_, sp, posTol))
+      launchCoop(kSweepLoop<R, 2, 3>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP, posIters_, sp, posTol, gb);
     KCHECK("position loop");
   }
   const bool posEmpty = useGS_ && posLeft == 0 && ncolP <= 0 && posIters_ > 0 && posTol > R(0);

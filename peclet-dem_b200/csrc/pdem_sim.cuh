@@ -405,12 +405,24 @@ class Sim {
     return e ? std::max(0L, std::strtol(e, nullptr, 10)) : 32768L;
   }();
   std::map<const void*, int> clusterOk_;  // per kernel: 1 resident, 0 not
-  // velocity-sweep records of the one-cluster loops (kPackPgs), packed once per substep
-  PgsRecs<R> packPgs(int nm, int ncol);
-  DBuf<Q4<R>> pgsQ_;
-  DBuf<int4> pgsIds_;
-  long pgsCap_ = 0;
-  long substepId_ = 0, pgsPackedAt_ = -1;
+  // the sweep loops as flows of body states (pdem_flow.cuh): records, links and mailboxes of the
+  // manifold and the contact colour orders
+  struct FlowBuf {
+    DBuf<char> rec;
+    DBuf<Q4<R>> var;
+    DBuf<R> lam;
+    DBuf<int> tab;
+    DBuf<uint4> box;
+    DBuf<unsigned> ctl;
+    unsigned tag = 0;       // largest tag a launch has used in the global mailboxes
+    long packedAt = -1;     // substep whose entries the records hold
+    int blocks = 0;         // blocks of the cluster the links address (0: global mailboxes)
+  };
+  FlowBuf flowM_, flowC_;
+  std::map<std::pair<const void*, int>, int> flowOk_;  // residency by (kernel, cluster blocks)
+  template <int KIND, int LOOP>
+  bool flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr);
+  long substepId_ = 0;
   // blocks of the one-cluster sweep loop (PDEM_SWEEP_CLUSTER: 8, the portable size, or 16, which
   // needs the non-portable cluster attribute) and the largest entry list it takes
   // (PDEM_SWEEP_CLUSTER_ENTRIES); larger lists sweep on the cooperative grid

@@ -225,11 +225,15 @@ __global__ void kVn0(Dev<R> d, int nm, R growthRate) {
 }
 
 // one-sided stabilization flags (src/solver_velocity.hpp:456-495)
+// order, flags (or null): the colour order and the flag word of its first entry (flagStride bytes from
+// one entry to the next), which takes the side flag too
 template <class R>
-__global__ void kSideFlags(Dev<R> d, int nm, V3<R> gHat, R riseThr, R approachThr) {
+__global__ void kSideFlags(Dev<R> d, int nm, V3<R> gHat, R riseThr, R approachThr, const int* order, char* flags,
+                           int flagStride, int sideShift) {
   if (!d.ctr->stabRun)
     return;
-  GRID_STRIDE(idx, nm) {
+  GRID_STRIDE(t, nm) {
+    const int idx = flags ? order[t] : (int)t;
     const uint8_t was = d.persistent[idx];
     d.sideFlags[idx] = 0;
     const int2 ab = d.mab[idx];
@@ -243,10 +247,15 @@ __global__ void kSideFlags(Dev<R> d, int nm, V3<R> gHat, R riseThr, R approachTh
     const V3<R> dx = sub(v3(d.posPred[ab.x]), v3(d.posPred[ab.y]));
     const R up = -(dx.x * gHat.x + dx.y * gHat.y + dx.z * gHat.z);
     const R thr = R(0.3) * sqrt(dot(dx, dx));
-    if (up > thr && -dot(v3(d.velPred[rb]), gHat) <= riseThr && d.grounded[rb] > 0)
+    if (up > thr && -dot(v3(d.velPred[rb]), gHat) <= riseThr && d.grounded[rb] > 0) {
       d.sideFlags[idx] = 1;
-    else if (up < -thr && -dot(v3(d.velPred[ra]), gHat) <= riseThr && d.grounded[ra] > 0)
+      if (flags)
+        *reinterpret_cast<int*>(flags + t * flagStride) |= 1 << sideShift;
+    } else if (up < -thr && -dot(v3(d.velPred[ra]), gHat) <= riseThr && d.grounded[ra] > 0) {
       d.sideFlags[idx] = 2;
+      if (flags)
+        *reinterpret_cast<int*>(flags + t * flagStride) |= 2 << sideShift;
+    }
   }
 }
 
@@ -404,87 +413,30 @@ __device__ __forceinline__ PgsStatic<R> pgsStatic(const Dev<R>& d, int idx) {
   s.wBn0 = s.Nsq * v.imB + genInvMass(v.TB, v.iIB, v.qB);
   return s;
 }
-// The records of a colour-ordered manifold list (PgsRecs), slot-major (slot k of entry t at
-// q[k * cap + t]): 0 (N, lenN), 1 (TA, Nsq), 2 (TB, wAn0), 3 (dc, wBn0), 4 (rAa, imA), 5 (rBa, imB),
-// 6 (wvN, eAvg), 7 (iIA, muAvg), 8 (iIB, 0), 9 qA, 10 qB; ids (manifold, ra, rb, hasB). A sweep
-// reads its entry's record with coalesced loads, then only the bodies' velocities depend on it.
-// Entries [0, coff[ncol]) of the colour order: the coloured manifolds.
+// The values one projected Gauss-Seidel update changes: the velocities and spins of its two bodies
+// (v1, w1 of a wall are not read) and its normal and tangential impulses.
 template <class R>
-__global__ void kPackPgs(Dev<R> d, const int* order, const int* coff, int ncol, PgsRecs<R> r) {
-  const long n = coff[ncol];
-  GRID_STRIDE(t, n) {
-    const int idx = order[t];
-    const PgsStatic<R> s = pgsStatic(d, idx);
-    const long c = r.cap;
-    r.q[t] = Q4<R>{s.N.x, s.N.y, s.N.z, s.lenN};
-    r.q[c + t] = Q4<R>{s.TA.x, s.TA.y, s.TA.z, s.Nsq};
-    r.q[2 * c + t] = Q4<R>{s.TB.x, s.TB.y, s.TB.z, s.wAn0};
-    r.q[3 * c + t] = Q4<R>{s.dc.x, s.dc.y, s.dc.z, s.wBn0};
-    r.q[4 * c + t] = Q4<R>{s.rAa.x, s.rAa.y, s.rAa.z, s.imA};
-    r.q[5 * c + t] = Q4<R>{s.rBa.x, s.rBa.y, s.rBa.z, s.imB};
-    r.q[6 * c + t] = Q4<R>{s.wvN.x, s.wvN.y, s.wvN.z, s.eAvg};
-    r.q[7 * c + t] = Q4<R>{s.iIA.x, s.iIA.y, s.iIA.z, s.muAvg};
-    r.q[8 * c + t] = Q4<R>{s.iIB.x, s.iIB.y, s.iIB.z, R(0)};
-    r.q[9 * c + t] = s.qA;
-    r.q[10 * c + t] = s.qB;
-    r.ids[t] = make_int4(idx, s.ra, s.rb, s.hasB ? 1 : 0);
-  }
-}
-template <class R>
-__device__ __forceinline__ PgsStatic<R> pgsRecord(const PgsRecs<R>& r, long t, int& idx) {
-  const long c = r.cap;
-  const int4 id = r.ids[t];
-  const Q4<R> a = r.q[t], b = r.q[c + t], e = r.q[2 * c + t], f = r.q[3 * c + t], g = r.q[4 * c + t],
-              h = r.q[5 * c + t], w = r.q[6 * c + t], ia = r.q[7 * c + t], ib = r.q[8 * c + t];
-  PgsStatic<R> s;
-  idx = id.x;
-  s.ra = id.y;
-  s.rb = id.z;
-  s.hasB = id.w != 0;
-  s.N = v3(a);
-  s.lenN = a.w;
-  s.TA = v3(b);
-  s.Nsq = b.w;
-  s.TB = v3(e);
-  s.wAn0 = e.w;
-  s.dc = v3(f);
-  s.wBn0 = f.w;
-  s.rAa = v3(g);
-  s.imA = g.w;
-  s.rBa = v3(h);
-  s.imB = h.w;
-  s.wvN = v3(w);
-  s.eAvg = w.w;
-  s.iIA = v3(ia);
-  s.muAvg = ia.w;
-  s.iIB = v3(ib);
-  s.qA = r.q[9 * c + t];
-  s.qB = r.q[10 * c + t];
-  return s;
-}
-
-// one projected Gauss-Seidel update of manifold idx from its per-substep constants v; with QS it
-// also raises *qs by the corrections of quasi-static contacts, |vn0| <= 4 vRest |N| (the residual
-// of the multilevel pass, src/solver_velocity.hpp:722-723, 829-830)
-template <class R, bool LOCAL = false, bool QS = false>
-__device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStatic<R>& v, R eG, R muG, int sc,
-                                        const SolveP<R>& P, R& mx, R* qs = nullptr) {
-  const int ra = v.ra, rb = v.rb;
+struct PgsVars {
+  V3<R> v0, w0, v1, w1;
+  R lam;
+  V3<R> lt;
+};
+// one projected Gauss-Seidel update from its per-substep constants v, side flag sf, approach velocity
+// vn0, position impulse and (read only with e_t != 0) approach tangential velocity vt0(): x in place,
+// every accepted correction to report(). Returns bit 0: lam changed, bit 1: lt changed, bit 2: the
+// update ran (the bodies' values are to be stored).
+template <class R, class VT0, class REPORT>
+__device__ __forceinline__ int pgsSolve(const PgsStatic<R>& v, int sf, R vn0, R posImp, VT0&& vt0, R eG, R muG,
+                                        const SolveP<R>& P, PgsVars<R>& x, REPORT&& report) {
   const bool hasB = v.hasB;
-  const V3<R> vA = v3(d.velPred[ra]), wA = v3(d.angVelPred[ra]);
-  V3<R> vB{0, 0, 0}, wB{0, 0, 0};
+  const V3<R> vA = x.v0, wA = x.w0;
+  V3<R> vB = hasB ? x.v1 : v.wvN, wB = hasB ? x.w1 : V3<R>{0, 0, 0};
   R e = eG;
-  if (hasB) {
-    vB = v3(d.velPred[rb]);
-    wB = v3(d.angVelPred[rb]);
-  } else {
-    vB = v.wvN;
-  }
   if (v.eAvg >= R(0))
     e = v.eAvg;
   const R lenN = v.lenN;
   if (lenN < R(1e-9))
-    return;
+    return 0;
   const V3<R> vG = mul(v.dc, P.growthRate);
   R vn = dot(vA, v.N) + dot(wA, v.TA) + dot(vB, neg(v.N)) + dot(wB, v.TB);
   vn += dot(vG, v.N);
@@ -493,7 +445,6 @@ __device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStati
   R wAn = v.wAn0;
   R wBn = v.wBn0;
   bool applyA = true, applyB = true;
-  const uint8_t sf = d.sideFlags[idx];
   if (sf == 1) {
     wBn = R(0);
     applyB = false;
@@ -505,25 +456,25 @@ __device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStati
   }
   const R wT = wAn + wBn;
   if (wT <= R(0))
-    return;
-  const R vn0 = d.vn0[idx];
+    return 0;
+  int changed = 4;
   const R v0 = sgn * vn0;
-  if (fabs(vn0) < P.vRest * lenN)
+  const bool slow = fabs(vn0) < P.vRest * lenN;
+  if (slow)
     e = R(0);
   const R target = (v0 > R(0)) ? -e * v0 : R(0);
   const R vt = sgn * vn;
   const R dp = (vt - target) / wT;
-  const R pOld = d.lambda[idx];
+  const R pOld = x.lam;
   R pNew = pOld + dp;
   if (pNew < R(0))
     pNew = R(0);
   const R dA = pNew - pOld;
   V3<R> vA2 = vA, wA2 = wA, vB2 = vB, wB2 = wB;
   if (dA != R(0)) {
-    d.lambda[idx] = pNew;
-    loopMax<R, LOCAL>(d, sc, false, fabs(dA) * wT / lenN, mx);
-    if (QS && fabs(vn0) <= R(4) * P.vRest * lenN)
-      runMax(*qs, fabs(dA) * wT / lenN);
+    x.lam = pNew;
+    changed |= 1;
+    report(fabs(dA) * wT / lenN);
     const R lam = -sgn * dA;
     const V3<R> J = mul(v.N, lam), JA = mul(v.TA, lam), JB = mul(v.TB, lam);
     if (applyA) {
@@ -539,7 +490,7 @@ __device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStati
   R mu = muG;
   if (v.muAvg >= R(0))
     mu = v.muAvg;
-  const V3<R> ltOld = v3(d.lambdaT[idx]);
+  const V3<R> ltOld = x.lt;
   const bool haveOld = nonzero(ltOld);
   if (mu > R(0) || haveOld) {
     const V3<R> nh = mul(v.N, R(1) / lenN);
@@ -548,11 +499,11 @@ __device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStati
     const V3<R> vr = sub(add(vA2, cross(wA2, v.rAa)), add(vBf, cross(wBf, v.rBa)));
     const V3<R> vtv = sub(vr, mul(nh, dot(vr, nh)));
     R beta = P.eT;
-    if (beta != R(0) && (sf != 0 || fabs(vn0) < P.vRest * lenN))
+    if (beta != R(0) && (sf != 0 || slow))
       beta = R(0);
     V3<R> err = vtv;
     if (beta != R(0)) {
-      V3<R> w0 = v3(d.vt0[idx]);
+      V3<R> w0 = vt0();
       w0 = sub(w0, mul(nh, dot(w0, nh)));
       err = add(vtv, mul(w0, beta));
     }
@@ -568,22 +519,20 @@ __device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStati
         ltNew = add(ltOld, mul(th, -vl / wTt));
     }
     ltNew = sub(ltNew, mul(nh, dot(ltNew, nh)));
-    R nTot = fmax(d.lambda[idx], R(0)) * lenN;
-    if (fabs(vn0) < P.vRest * lenN)
-      nTot += fmax(d.posImp[idx], R(0));
+    R nTot = fmax(x.lam, R(0)) * lenN;
+    if (slow)
+      nTot += fmax(posImp, R(0));
     const R bound = mu * nTot;
     const R ll = sqrt(dot(ltNew, ltNew));
     if (ll > bound)
       ltNew = (bound > R(0)) ? mul(ltNew, bound / ll) : V3<R>{0, 0, 0};
     const V3<R> dd = sub(ltNew, ltOld);
     if (nonzero(dd)) {
-      d.lambdaT[idx] = q4(ltNew);
+      x.lt = ltNew;
+      changed |= 2;
       const R dl = sqrt(dot(dd, dd));
-      if (wTt > R(1e-9)) {
-        loopMax<R, LOCAL>(d, sc, false, dl * wTt, mx);
-        if (QS && fabs(vn0) <= R(4) * P.vRest * lenN)
-          runMax(*qs, dl * wTt);
-      }
+      if (wTt > R(1e-9))
+        report(dl * wTt);
       if (applyA) {
         vA2 = add(vA2, mul(dd, v.imA));
         wA2 = add(wA2, angResponse(v.qA, cross(v.rAa, dd), v.iIA));
@@ -594,11 +543,48 @@ __device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStati
       }
     }
   }
-  d.velPred[ra] = q4(vA2);
-  d.angVelPred[ra] = q4(wA2);
+  x.v0 = vA2;
+  x.w0 = wA2;
   if (hasB) {
-    d.velPred[rb] = q4(vB2);
-    d.angVelPred[rb] = q4(wB2);
+    x.v1 = vB2;
+    x.w1 = wB2;
+  }
+  return changed;
+}
+// the same update on the manifold's global state; with QS it also raises *qs by the corrections of
+// quasi-static contacts, |vn0| <= 4 vRest |N| (the residual of the multilevel pass,
+// src/solver_velocity.hpp:722-723, 829-830)
+template <class R, bool LOCAL = false, bool QS = false>
+__device__ __forceinline__ void pgsCore(const Dev<R>& d, int idx, const PgsStatic<R>& v, R eG, R muG, int sc,
+                                        const SolveP<R>& P, R& mx, R* qs = nullptr) {
+  PgsVars<R> x;
+  x.v0 = v3(d.velPred[v.ra]);
+  x.w0 = v3(d.angVelPred[v.ra]);
+  x.v1 = x.w1 = V3<R>{0, 0, 0};
+  if (v.hasB) {
+    x.v1 = v3(d.velPred[v.rb]);
+    x.w1 = v3(d.angVelPred[v.rb]);
+  }
+  x.lam = d.lambda[idx];
+  x.lt = v3(d.lambdaT[idx]);
+  const R vn0 = d.vn0[idx];
+  const int changed = pgsSolve<R>(v, d.sideFlags[idx], vn0, d.posImp[idx], [&] { return v3(d.vt0[idx]); }, eG, muG, P,
+                                  x, [&](R m) {
+                                    loopMax<R, LOCAL>(d, sc, false, m, mx);
+                                    if (QS && fabs(vn0) <= R(4) * P.vRest * v.lenN)
+                                      runMax(*qs, m);
+                                  });
+  if (!changed)
+    return;
+  if (changed & 1)
+    d.lambda[idx] = x.lam;
+  if (changed & 2)
+    d.lambdaT[idx] = q4(x.lt);
+  d.velPred[v.ra] = q4(x.v0);
+  d.angVelPred[v.ra] = q4(x.w0);
+  if (v.hasB) {
+    d.velPred[v.rb] = q4(x.v1);
+    d.angVelPred[v.rb] = q4(x.w1);
   }
 }
 

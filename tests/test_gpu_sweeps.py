@@ -1,0 +1,63 @@
+"""The sweep loops' launch forms against the oracle, at the sizes where they change: the flow of body
+states in one cluster (1 to 16 blocks) and on the grid, ragged last warps, single bodies, a body in
+contact with its own periodic image, an adaptive stop after the first sweep and one sweep only. Bit-exact at
+float; 1e-12 relative at double, the step's own bar."""
+import numpy as np
+import pytest
+
+import parity as P
+from peclet.dem import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+PRECISIONS = [("fp32", 0.0), ("fp64", 1e-12)]
+
+
+def _compare(gpu_api, orc_api, sc, steps, precision, rtol):
+    a, b = P.build(gpu_api, sc, None, precision), P.build(orc_api, sc, None, precision)
+    for k in range(steps):
+        a.step(sc.dt)
+        b.step(sc.dt)
+        bad = P.diff(P.snapshot(a), P.snapshot(b), rtol=rtol)
+        assert not bad, f"substep {k}: {bad[:4]}"
+    return a
+
+
+def _bed(n, iters=(10, 10), seed=41):
+    """The first n spheres of a touching lattice column on the floor."""
+    nx = max(1, round(n ** (1 / 3)))
+    sc = W.plain_settling(seed=seed, nx=nx, ny=nx, nz=-(-n // (nx * nx)), cells_z=n // (nx * nx) + 3, spacing_r=1.98,
+                          jitter_r=0.02, vmax=0.05, iterations=iters)
+    sc.pos, sc.vel, sc.inv_mass, sc.inv_inertia = (a[:n].copy() for a in (sc.pos, sc.vel, sc.inv_mass, sc.inv_inertia))
+    return sc
+
+
+@pytest.mark.parametrize("precision,rtol", PRECISIONS)
+@pytest.mark.parametrize("entries", [None, 0], ids=["cluster", "grid"])
+@pytest.mark.parametrize("n,iters", [(1, (10, 10)), (2, (10, 10)), (65, (1, 1)), (700, (3, 10)), (2500, (10, 4))])
+def test_flow_forms(gpu_api, orc_api, monkeypatch, n, iters, entries, precision, rtol):
+    if entries is not None:
+        monkeypatch.setenv("PDEM_SWEEP_CLUSTER_ENTRIES", str(entries))
+    _compare(gpu_api, orc_api, _bed(n, iters), 3, precision, rtol)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_flow_own_image(gpu_api, monkeypatch, precision):
+    """Spheres stacked in a box periodic in x that is narrower than a sphere: each touches its own image
+    (one body on both sides of a manifold). The cluster and the grid give the same bits."""
+    r, L = 1e-3, 1.995e-3
+    rng = np.random.default_rng(3)
+    pos = np.stack([np.full(5, 0.5 * L), np.full(5, r), r * (0.99 + 1.98 * np.arange(5))], 1)
+    im, inertia = W.sphere_props(r, 2500.0)
+    sc = W.Scene(name="own_image", pos=pos, vel=rng.uniform(-0.05, 0.05, (5, 3)), inv_mass=np.full(5, im),
+                 inv_inertia=np.full((5, 3), inertia), global_scale=r,
+                 domain=((0, 0, 0), (L, 3 * r, 14 * r), (True, False, False)), planes=[(0, 0, 0, 0, 0, 1)],
+                 material=(0.5, 0.0, 0.5), dt=1e-5)
+    a = P.build(gpu_api, sc, None, precision)
+    monkeypatch.setenv("PDEM_SWEEP_CLUSTER_ENTRIES", "0")
+    b = P.build(gpu_api, sc, None, precision)
+    for _ in range(4):
+        a.step(sc.dt)
+        b.step(sc.dt)
+        assert not P.diff(P.snapshot(a), P.snapshot(b))
+    assert a.counters()["manifolds"] > 5
