@@ -10,6 +10,7 @@
 
 #include "pdem_broad.cuh"
 #include "pdem_contact.cuh"
+#include "pdem_dense.cuh"
 #include "pdem_flow.cuh"
 #include "pdem_hertz.cuh"
 #include "pdem_kernels.cuh"
@@ -494,6 +495,56 @@ static int bitsFor(long maxValue) {
   while (b < 64 && (1L << b) <= maxValue)
     ++b;
   return b;
+}
+
+// The position sweeps of a contact graph with saturated or uncoloured contacts (pdem_dense.cuh). One
+// block while the bodies' positions fit its shared memory and the contacts are few enough for one SM,
+// else the cooperative grid.
+template <class R>
+void Sim<R>::denseSweeps(int nc, int ncol, int left, R tol) {
+  cudaStream_t s = stream_;
+  const int nb = numParticles_;
+  denseQ_.ensure(3 * (size_t)nc, false, s);
+  denseIds_.ensure((size_t)nc, false, s);
+  const DenseRecs<R> rec{denseQ_.p, denseIds_.p, (long)nc};
+  ++launches_, kDensePack<R><<<gridFor(nc), kBlock, 0, s>>>(d_, cOrder_.p, nc, rec);
+  KCHECK("dense records");
+  const size_t n1 = (size_t)nc + 2;
+  denseRuns_.ensure(5 * n1 + (size_t)nb + 2, false, s);
+  int* p = denseRuns_.p;
+  const DenseRuns D{p, p + n1, p + 3 * n1, p + 4 * n1, p + 5 * n1, p + 5 * n1 + nb};
+  if (ncol > kSaturatedColor) {
+    ++launches_, kDenseRuns<R><<<1, 1024, 0, s>>>(d_, cOrder_.p, cOff_.p, nb, D);
+    KCHECK("dense runs");
+  }
+  if (left > 0) {  // incidence lists of the uncoloured contacts, in contact order
+    incKind_ = -1;
+    incKeys_.ensure(2 * (size_t)left, false, s);
+    incKeysS_.ensure(2 * (size_t)left, false, s);
+    incVals_.ensure(2 * (size_t)left, false, s);
+    incValsS_.ensure(2 * (size_t)left, false, s);
+    incOff_.ensure((size_t)nb + 2, false, s);
+    qA_.ensure(left, false, s);
+    iC_.ensure(left, false, s);
+    ++launches_, kDenseLeftKeys<R><<<gridFor(left), kBlock, 0, s>>>(d_, cOrder_.p, nc - left, left, incKeys_.p, incVals_.p, nb);
+    sortPairs(incKeys_.p, incKeysS_.p, incVals_.p, incValsS_.p, 2 * left, bitsFor(nb));
+    ++launches_, kLowerBoundOffsets<int><<<gridFor(nb + 1), kBlock, 0, s>>>(2 * left, incKeysS_.p, nb, incOff_.p);
+    KCHECK("dense incidence");
+  }
+  const Incidence inc{incOff_.p, incValsS_.p};
+  gbar_.ensure(2, false, s);
+  const GridBar gb{gbar_.p, &ctr_.p->err, barrierSleepNs_, barrierSpins_};
+  ctl(CTL_POS_BEGIN, R(0), 0);
+  const size_t smem = (size_t)nb * sizeof(Q4<R>);
+  if (smem <= kDenseMaxSmem && nc <= denseOneEntries_) {
+    auto* k = kDenseSweeps<R, true>;
+    cudaCheck(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseMaxSmem), "smem attribute");
+    ++launches_, k<<<1, kDenseBlock, smem, s>>>(d_, cOff_.p, ncol, posIters_, tol, gb, rec, D, nb, left, inc, qA_.p, iC_.p);
+  } else {
+    launchCoopB(kDenseSweeps<R, false>, kDenseBlock, d_, (const int*)cOff_.p, ncol, posIters_, tol, gb, rec, D, nb, left,
+                inc, qA_.p, iC_.p);
+  }
+  KCHECK("dense sweeps");
 }
 
 // =============================================================================================
@@ -1909,14 +1960,18 @@ void Sim<R>::demStep() {
   const R posTol = R(1e-4) * baseRadius_ * gs_;
   if (nc > 0)
     posLamC_.zero(s, nc);
-  const bool posJacobi = (posLeft > 0 || !useGS_) && nc > 0;
+  // contacts the 62 colours do not hold (pdem_dense.cuh)
+  const bool posDense = useGS_ && !batch_ && nc > 0 && posIters_ > 0 && (posLeft > 0 || ncolP > kSaturatedColor);
+  const bool posJacobi = !useGS_ && nc > 0;
+  if (posDense)
+    denseSweeps(nc, ncolP, posLeft, posTol);
   if (posJacobi) {
     buildIncidence(2, nc, numParticles_);
     qA_.ensure(nc, false, s);
     iC_.ensure(nc, false, s);
   }
   Incidence incP{incOff_.p, incValsS_.p};
-  const bool posPersistent = useGS_ && posLeft == 0 && ncolP > 0 && posIters_ > 0;
+  const bool posPersistent = useGS_ && !posDense && ncolP > 0 && posIters_ > 0;
   if (posPersistent) {
     gbar_.ensure(2, false, s);
     const GridBar gb{gbar_.p, &ctr_.p->err, barrierSleepNs_, barrierSpins_};
@@ -1929,28 +1984,21 @@ void Sim<R>::demStep() {
       launchCoop(kSweepLoop<R, 2, 3>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP, posIters_, sp, posTol, gb);
     KCHECK("position loop");
   }
-  const bool posEmpty = useGS_ && posLeft == 0 && ncolP <= 0 && posIters_ > 0 && posTol > R(0);
+  const bool posEmpty = useGS_ && !posDense && ncolP <= 0 && posIters_ > 0 && posTol > R(0);
   if (posEmpty) {  // as velEmpty: maxOverlap = 0 < posTol ends the loop after its first sweep
     ctl(CTL_POS_BEGIN, R(0), 0);
     ctl(CTL_POS_END, posTol, 0);
   }
-  for (int it = 0; it < (posPersistent || posEmpty ? 0 : posIters_); ++it) {
-    if (useGS_) {
+  for (int it = 0; it < (posDense || posPersistent || posEmpty ? 0 : posIters_); ++it) {
+    if (useGS_) {  // nothing to sweep, and a tolerance that ends no loop
       ctl(CTL_POS_BEGIN, R(0), 0);
-      for (int col = 0; col < ncolP; ++col)
-        ++launches_, kPosGSColor<<<gridFor(nc), B, 0, s>>>(d_, cOrder_.p, cOff_.p, col, 3);
-      if (posLeft > 0) {
-        ++launches_, kPosJacobiPre<<<gridFor(nc), B, 0, s>>>(d_, nc, 1, qA_.p, iC_.p, 3);
-        ++launches_, kPosJacobiGather<<<gridFor(numParticles_), B, 0, s>>>(d_, numParticles_, incP, qA_.p, iC_.p, 3);
-        ++launches_, kApplyUpdatesGated<<<gridFor(numParticles_), B, 0, s>>>(d_, numParticles_, 3);
-      }
       ctl(CTL_POS_END, posTol, 0);
     } else {
       if (nc > 0) {
-        ++launches_, kPosJacobiPre<<<gridFor(nc), B, 0, s>>>(d_, nc, 0, qA_.p, iC_.p, 0);
-        ++launches_, kPosJacobiGather<<<gridFor(numParticles_), B, 0, s>>>(d_, numParticles_, incP, qA_.p, iC_.p, 0);
+        ++launches_, kPosJacobiPre<<<gridFor(nc), B, 0, s>>>(d_, nc, qA_.p, iC_.p);
+        ++launches_, kPosJacobiGather<<<gridFor(numParticles_), B, 0, s>>>(d_, numParticles_, incP, qA_.p, iC_.p);
       }
-      ++launches_, kApplyUpdatesGated<<<gridFor(numParticles_), B, 0, s>>>(d_, numParticles_, 0);
+      ++launches_, kApplyUpdates<<<gridFor(numParticles_), B, 0, s>>>(d_, numParticles_);
     }
     KCHECK("position sweep");
   }

@@ -422,6 +422,15 @@ class Sim {
   std::map<std::pair<const void*, int>, int> flowOk_;  // residency by (kernel, cluster blocks)
   template <int KIND, int LOOP>
   bool flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr);
+  void denseSweeps(int nc, int ncol, int left, R tol);
+  DBuf<Q4<R>> denseQ_;
+  DBuf<int4> denseIds_;
+  DBuf<int> denseRuns_;
+  // most contacts whose dense sweeps run in one block (PDEM_DENSE_ONE_ENTRIES)
+  long denseOneEntries_ = [] {
+    const char* e = std::getenv("PDEM_DENSE_ONE_ENTRIES");
+    return e ? std::max(0L, std::strtol(e, nullptr, 10)) : 1L << 18;
+  }();
   long substepId_ = 0;
   // blocks of the one-cluster sweep loop (PDEM_SWEEP_CLUSTER: 8, the portable size, or 16, which
   // needs the non-portable cluster attribute) and the largest entry list it takes

@@ -1113,36 +1113,12 @@ __device__ __forceinline__ void posGSOne(const Dev<R>& d, int idx, R& mx) {
   }
   loopMax<R, LOCAL>(d, sc, true, -C, mx);
 }
-template <class R>
-__global__ void kPosGSColor(Dev<R> d, const int* order, const int* coff, int color, int gate) {
-  if (!gateOpen(d.ctr, gate))
-    return;
-  const int b = coff[color], n = coff[color + 1] - b;
-  // colour 62 is where the 62-colour mask saturates: it is not an independent set, so it
-  // runs serially in manifold order, as the reference's serial sweep does
-  const bool serial = color >= kSaturatedColor;
-  if (serial && (blockIdx.x | threadIdx.x))
-    return;
-  R mx = R(0);
-  for (long t = serial ? 0 : (long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += serial ? 1 : (long)gridDim.x * blockDim.x) {
-    posGSOne(d, order[b + t], mx);
-  }
-  if (serial)
-    atomicMaxNonNeg(&d.ctr->maxOverlap, mx);
-  else
-    warpMaxAtomic(&d.ctr->maxOverlap, mx);
-}
 // Jacobi position solve (src/solver_position.hpp:34-134): per-contact correction pre-pass, then a
 // gather per body slot in contact order
 template <class R>
-__global__ void kPosJacobiPre(Dev<R> d, int nc, int filt, Q4<R>* corr, int* ok, int gate) {
-  if (!gateOpen(d.ctr, gate))
-    return;
+__global__ void kPosJacobiPre(Dev<R> d, int nc, Q4<R>* corr, int* ok) {
   GRID_STRIDE(idx, nc) {
     ok[idx] = 0;
-    if (filt && d.cColor[idx] != -1)
-      continue;
     V3<R> nv;
     R C = R(0), wT = R(0);
     int A, B;
@@ -1158,9 +1134,7 @@ __global__ void kPosJacobiPre(Dev<R> d, int nc, int filt, Q4<R>* corr, int* ok, 
   }
 }
 template <class R>
-__global__ void kPosJacobiGather(Dev<R> d, int n, Incidence inc, const Q4<R>* corr, const int* ok, int gate) {
-  if (!gateOpen(d.ctr, gate))
-    return;
+__global__ void kPosJacobiGather(Dev<R> d, int n, Incidence inc, const Q4<R>* corr, const int* ok) {
   GRID_STRIDE(b, n) {
     const int s = inc.off[b], e = inc.off[b + 1];
     if (s == e)
@@ -1184,23 +1158,6 @@ __global__ void kPosJacobiGather(Dev<R> d, int n, Incidence inc, const Q4<R>* co
     d.counts[b] = cnt;
   }
 }
-template <class R>
-__global__ void kApplyUpdatesGated(Dev<R> d, int n, int gate) {
-  if (!gateOpen(d.ctr, gate))
-    return;
-  GRID_STRIDE(i, n) {
-    const int c = d.counts[i];
-    if (c <= 0)
-      continue;
-    const R f = R(1) / static_cast<R>(c);
-    d.posPred[i] = q4(add(v3(d.posPred[i]), mul(v3(d.dPos[i]), f)));
-    d.velPred[i] = q4(add(v3(d.velPred[i]), mul(v3(d.dVel[i]), f)));
-    d.dPos[i] = Q4<R>{0, 0, 0, 0};
-    d.dVel[i] = Q4<R>{0, 0, 0, 0};
-    d.counts[i] = 0;
-  }
-}
-
 // incidence entries: entry 2i = (body of side A, i<<1), 2i+1 = (body of side B, i<<1|1) or none
 template <class R, int KIND>
 __global__ void kIncidenceKeys(Dev<R> d, int ne, int* keys, int* vals, int none) {

@@ -1,11 +1,13 @@
 """The sweep loops' launch forms against the oracle, at the sizes where they change: the flow of body
 states in one cluster (1 to 16 blocks) and on the grid, ragged last warps, single bodies, a body in
-contact with its own periodic image, an adaptive stop after the first sweep and one sweep only. Bit-exact at
+contact with its own periodic image, an adaptive stop after the first sweep and one sweep only; and the
+dense position sweeps (saturated and uncoloured contacts) in one block and on the grid. Bit-exact at
 float; 1e-12 relative at double, the step's own bar."""
 import numpy as np
 import pytest
 
 import parity as P
+import scenes as S
 from peclet.dem import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +63,29 @@ def test_flow_own_image(gpu_api, monkeypatch, precision):
         b.step(sc.dt)
         assert not P.diff(P.snapshot(a), P.snapshot(b))
     assert a.counters()["manifolds"] > 5
+
+
+def _stacked(n, points, seed=7):
+    """Hollow cylinders side by side with a small tilt: tens of shell-point contacts a pair."""
+    rng = np.random.default_rng(seed)
+    nx = max(2, round(n ** (1 / 3)))
+    pitch = np.array([2.0e-3, 3.1e-3, 2.0e-3])
+    k = np.arange(n)
+    sc = S.cylinders(seed=seed, n=n, shell=W.hollow_cylinder_shell(points, seed=seed))
+    sc.pos = (np.stack([k % nx, k // (nx * nx), (k // nx) % nx], 1) + 0.5) * pitch + rng.uniform(-1e-5, 1e-5, (n, 3))
+    half, spin = rng.normal(0.0, 0.005, (n, 2)), rng.uniform(0.0, np.pi, n)
+    sc.quat = np.stack([half[:, 0], np.sin(spin), half[:, 1], np.cos(spin)], 1)
+    sc.quat /= np.linalg.norm(sc.quat, axis=1, keepdims=True)
+    mx = tuple(np.array([nx, n // (nx * nx) + 1, nx]) * pitch)
+    sc.domain, sc.planes = ((0, 0, 0), mx, (False,) * 3), W.box_planes((0, 0, 0), mx)
+    return sc
+
+
+@pytest.mark.parametrize("precision,rtol", PRECISIONS)
+@pytest.mark.parametrize("entries", [None, 0], ids=["block", "grid"])
+@pytest.mark.parametrize("n,points,colours", [(2, 512, 0), (9, 256, 0), (120, 512, 63)])
+def test_dense_forms(gpu_api, orc_api, monkeypatch, n, points, colours, entries, precision, rtol):
+    if entries is not None:
+        monkeypatch.setenv("PDEM_DENSE_ONE_ENTRIES", str(entries))
+    sim = _compare(gpu_api, orc_api, _stacked(n, points), 2, precision, rtol)
+    assert sim.counters()["colors_position"] >= colours
