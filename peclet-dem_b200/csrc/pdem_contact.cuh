@@ -972,11 +972,6 @@ __device__ __forceinline__ void groundSweepsWarp(int nm, int b0, int nb, int swe
   for (int i = lane; i < nb; i += 32)
     grounded[b0 + i] = (uint8_t)L[i];
 }
-__global__ void kGroundSweeps(int nm, int numReal, int sweeps, const int4* edges, uint8_t* grounded,
-                              int* gscratch, int useShared) {
-  extern __shared__ int slvl[];
-  groundSweepsWarp(nm, 0, numReal, sweeps, edges, grounded, useShared ? slvl : gscratch);
-}
 // The same support levels from the least fixed point, in parallel. The serial sweeps only raise
 // levels, each raise is an edge relaxation (wall: 255; support: the source's level - 1 when
 // positive), so they climb towards the least fixed point F above the decayed levels L0, the same

@@ -220,6 +220,98 @@ __global__ void __launch_bounds__(kSceneBlockMax) kSweepScenes(Dev<R> d, const i
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// kGroundLevels on the whole grid, for graphs whose levels, times and edges do not fit one block's
+// shared memory (about 5,600 spheres in a bed): the same relaxations of the levels L and times T, in
+// global memory, the passes behind the grid barrier. A pass relaxes every edge kGroundInner times, so
+// that support chains advance between barriers. The one warp that ran the exact serial sweeps of such
+// graphs before needs 1.4 ms a substep on 20,011 spheres (61,000 manifolds); it remains for the graphs
+// that do not reach the fixed point within the serial sweeps' count.
+// ctl: [0..2] a pass changed something (pass % 3), [3] some body late; zero before the launch.
+constexpr int kGroundInner = 4;
+static __global__ void __launch_bounds__(kGroundBlock) kGroundLevelsGrid(int nm, int nb, int sweeps, const int4* edges,
+                                                                        uint8_t* grounded, int* L, u64* T, int* ctl,
+                                                                        GridBar gb) {
+  volatile int* VL = L;
+  volatile u64* VT = T;
+  volatile int* VC = ctl;
+  const long gtid = (long)blockIdx.x * blockDim.x + threadIdx.x, gstride = (long)gridDim.x * blockDim.x;
+  const bool lead = gtid == 0;
+  const u64 kInf = ~0ull, kStart = 1ull << 32;  // (sweep << 32) | (edge + 1); 1 << 32: final before sweep 1
+  for (long i = gtid; i < nb; i += gstride)
+    L[i] = grounded[i];
+  if (!gridBarrier(gb))
+    return;
+  int pass = 0;
+  // passes of relax(edge index, edge) -> changed, until one changes nothing; 1: done, 0: too many
+  // passes, -1: a barrier timed out
+  auto settle = [&](auto relax) -> int {
+    for (int k = 0; k < kGroundPassCap; ++k, ++pass) {
+      int ch = 0;
+      for (int q = 0; q < kGroundInner; ++q)
+        for (long e = gtid; e < nm; e += gstride)
+          ch |= relax(e, edges[e]) ? 1 : 0;
+      if (__syncthreads_or(ch) && threadIdx.x == 0)
+        VC[pass % 3] = 1;
+      if (!gridBarrier(gb))
+        return -1;
+      const int any = VC[pass % 3];
+      if (lead)
+        VC[(pass + 2) % 3] = 0;  // read by every block before it arrived here
+      if (!any) {
+        ++pass;
+        return 1;
+      }
+    }
+    return 0;
+  };
+  int ok = settle([&](long, const int4& g) {  // (a) F
+    const int c = g.x == 1 ? 255 : (g.x == 2 ? VL[g.y] - 1 : 0);
+    if (c > 0 && c > VL[g.z]) {
+      atomicMax(&L[g.z], c);
+      return true;
+    }
+    return false;
+  });
+  if (ok < 0)
+    return;
+  for (long i = gtid; i < nb; i += gstride)
+    T[i] = VL[i] == (int)grounded[i] ? kStart : kInf;
+  if (!gridBarrier(gb))
+    return;
+  if (ok > 0)
+    ok = settle([&](long e, const int4& g) {  // (b) the sweep in which each body becomes final
+      u64 te = kInf;
+      if (g.x == 1 && VL[g.z] == 255) {
+        te = kStart | (u64)(e + 1);
+      } else if (g.x == 2 && VL[g.z] > 0 && VL[g.y] - 1 == VL[g.z]) {
+        const u64 tu = VT[g.y];
+        if (tu != kInf)
+          te = (((e > (long)(tu & 0xffffffffull) - 1 ? tu >> 32 : (tu >> 32) + 1)) << 32) | (u64)(e + 1);
+      }
+      if (te < VT[g.z]) {
+        atomicMin(&T[g.z], te);
+        return true;
+      }
+      return false;
+    });
+  if (ok < 0)
+    return;
+  int late = !ok;
+  for (long i = gtid; i < nb && !late; i += gstride)
+    late = VT[i] == kInf || (VT[i] >> 32) > (u64)sweeps;
+  if (__syncthreads_or(late) && threadIdx.x == 0)
+    VC[3] = 1;
+  if (!gridBarrier(gb))
+    return;
+  if (!VC[3]) {  // (c)
+    for (long i = gtid; i < nb; i += gstride)
+      grounded[i] = (uint8_t)VL[i];
+  } else if (blockIdx.x == 0 && threadIdx.x < 32) {
+    groundSweepsWarp(nm, 0, nb, sweeps, edges, grounded, L);
+  }
+}
+
 constexpr int kColorBlock = 1024;  // one large block per SM: fewer arrivals per grid barrier
 
 // ---------------------------------------------------------------------------------------------

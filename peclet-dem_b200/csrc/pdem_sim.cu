@@ -2687,7 +2687,6 @@ void Sim<R>::ensureGrounded() {
   }
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(kGroundSweeps, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(kGroundSweepsScenes, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(kGroundLevels, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     attr = true;
@@ -2705,15 +2704,24 @@ void Sim<R>::ensureGrounded() {
         gscratch_.ensure(nr, false, stream_);
       ++launches_, kGroundSweepsScenes<<<S, 32, smem ? maxSceneBodies_ * sizeof(int) : 0, stream_>>>(
           gRingScn_[slot].p, sceneFirstD_.p, 8, gRing_[slot].p, grounded_.p, gscratch_.p, smem);
-    } else if (nm > 0 && (size_t)nr * 12 + (size_t)nm * 8 <= 200 * 1024 && nr < (1 << 30)) {
+    } else if (nm > 0 && (size_t)nr * 12 + (size_t)nm * 8 <= groundOneBytes_ && nr < (1 << 30)) {
       ++launches_, kGroundLevels<<<1, kGroundBlock, (size_t)nr * 12 + (size_t)nm * 8, stream_>>>(
           nm, nr, 8, gRing_[slot].p, grounded_.p);
     } else if (nm > 0) {
-      const bool smem = (size_t)nr * sizeof(int) <= 200 * 1024;
-      if (!smem)
-        gscratch_.ensure(nr, false, stream_);
-      ++launches_, kGroundSweeps<<<1, 32, smem ? nr * sizeof(int) : 0, stream_>>>(nm, nr, 8, gRing_[slot].p,
-                                                                                grounded_.p, gscratch_.p, smem);
+      gscratch_.ensure(nr, false, stream_);
+      groundT_.ensure(nr, false, stream_);
+      groundCtl_.ensure(4, false, stream_);
+      groundCtl_.zero(stream_);
+      gbar_.ensure(2, false, stream_);
+      gbar_.zero(stream_);
+      const GridBar gb{gbar_.p, &ctr_.p->err, 0u, barrierSpins_};
+      const int grid = std::min(coopGrid(kGroundLevelsGrid, kGroundBlock), (std::max(nm, nr) + kGroundBlock - 1) / kGroundBlock);
+      int nmA = nm, nrA = nr, sweeps = 8;
+      const int4* edges = gRing_[slot].p;
+      void* argv[] = {&nmA, &nrA, &sweeps, &edges, &grounded_.p, &gscratch_.p, &groundT_.p, &groundCtl_.p, const_cast<GridBar*>(&gb)};
+      ++launches_;
+      cudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kGroundLevelsGrid), dim3(grid), dim3(kGroundBlock),
+                                            argv, 0, stream_), "support levels (grid)");
     }
     KCHECK("support sweeps");
   }

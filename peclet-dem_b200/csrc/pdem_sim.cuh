@@ -307,7 +307,13 @@ class Sim {
   int gRingScenes_[kGroundRing] = {};   // batched form: scenes of the slot (0: one scene)
   DBuf<int> gRingScn_[kGroundRing];     // batched form: first manifold of each scene in the slot
   long gLog_ = 0, gCheckpoint_ = 0;
-  DBuf<int> gscratch_;
+  DBuf<int> gscratch_, groundCtl_;
+  DBuf<u64> groundT_;
+  // shared memory up to which one block computes the support levels (PDEM_GROUND_ONE_BYTES)
+  size_t groundOneBytes_ = [] {
+    const char* e = std::getenv("PDEM_GROUND_ONE_BYTES");
+    return e ? (size_t)std::min(std::max(0L, std::strtol(e, nullptr, 10)), 200L * 1024) : (size_t)200 * 1024;
+  }();
   DBuf<double> thermo_;
   // broadphase scratch
   DBuf<char> bvhBoxes_, bvhNodes_;

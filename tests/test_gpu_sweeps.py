@@ -89,3 +89,12 @@ def test_dense_forms(gpu_api, orc_api, monkeypatch, n, points, colours, entries,
         monkeypatch.setenv("PDEM_DENSE_ONE_ENTRIES", str(entries))
     sim = _compare(gpu_api, orc_api, _stacked(n, points), 2, precision, rtol)
     assert sim.counters()["colors_position"] >= colours
+
+
+@pytest.mark.parametrize("precision,rtol", PRECISIONS)
+@pytest.mark.parametrize("scene", ["bed", "reversed"])
+def test_support_levels_on_the_grid(gpu_api, orc_api, monkeypatch, scene, precision, rtol):
+    """The support levels computed by the whole grid (every graph sent there): a bed whose serial sweeps
+    reach the fixed point, and a column numbered top to bottom whose sweeps stop short of it."""
+    monkeypatch.setenv("PDEM_GROUND_ONE_BYTES", "0")
+    _compare(gpu_api, orc_api, _bed(700) if scene == "bed" else S.reversed_column(), 12, precision, rtol)
