@@ -84,7 +84,6 @@ struct Dev {
   R *invMass = nullptr, *scale = nullptr, *targetScale = nullptr, *rad = nullptr, *planeFric = nullptr;
   int *shapeId = nullptr, *realIdx = nullptr, *counts = nullptr;
   uint8_t *grounded = nullptr, *matId = nullptr;
-  long long* winner = nullptr;
   u64* mask = nullptr;
   int2* pairs = nullptr;
   // contacts

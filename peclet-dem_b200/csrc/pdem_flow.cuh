@@ -92,22 +92,6 @@ __device__ __forceinline__ uint4 flowLoadShared(unsigned addr) {
       : "memory");
   return v;
 }
-__device__ __forceinline__ void flowStoreGlobal(uint4* p, unsigned x, unsigned y, unsigned z, unsigned w) {
-  asm volatile(
-      "{\n .reg .b128 q;\n .reg .b64 lo, hi;\n mov.b64 lo, {%1, %2};\n mov.b64 hi, {%3, %4};\n mov.b128 q, {lo, hi};\n"
-      " st.relaxed.gpu.global.b128 [%0], q;\n}" ::"l"(p), "r"(x), "r"(y), "r"(z), "r"(w)
-      : "memory");
-}
-__device__ __forceinline__ uint4 flowLoadGlobal(const uint4* p) {
-  uint4 v;
-  asm volatile(
-      "{\n .reg .b128 q;\n .reg .b64 lo, hi;\n ld.relaxed.gpu.global.b128 q, [%4];\n mov.b128 {lo, hi}, q;\n"
-      " mov.b64 {%0, %1}, lo;\n mov.b64 {%2, %3}, hi;\n}"
-      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-      : "l"(p)
-      : "memory");
-  return v;
-}
 __device__ __forceinline__ unsigned flowRemoteAddr(unsigned local, int rank) {
   unsigned r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));

@@ -312,45 +312,68 @@ static __global__ void __launch_bounds__(kGroundBlock) kGroundLevelsGrid(int nm,
   }
 }
 
+// 128-bit single-copy atomic accesses
+__device__ __forceinline__ void flowStoreGlobal(uint4* p, unsigned x, unsigned y, unsigned z, unsigned w) {
+  asm volatile(
+      "{\n .reg .b128 q;\n .reg .b64 lo, hi;\n mov.b64 lo, {%1, %2};\n mov.b64 hi, {%3, %4};\n mov.b128 q, {lo, hi};\n"
+      " st.relaxed.gpu.global.b128 [%0], q;\n}" ::"l"(p), "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
+__device__ __forceinline__ uint4 flowLoadGlobal(const uint4* p) {
+  uint4 v;
+  asm volatile(
+      "{\n .reg .b128 q;\n .reg .b64 lo, hi;\n ld.relaxed.gpu.global.b128 q, [%4];\n mov.b128 {lo, hi}, q;\n"
+      " mov.b64 {%0, %1}, lo;\n mov.b64 {%2, %3}, hi;\n}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p)
+      : "memory");
+  return v;
+}
+
 constexpr int kColorBlock = 1024;  // one large block per SM: fewer arrivals per grid barrier
 
 // ---------------------------------------------------------------------------------------------
-// Both colourings of a substep in ONE cooperative launch: the manifold graph (velocity solve) and
-// the contact graph (position solve) are independent, so their Jones-Plassmann rounds run in
-// lockstep behind the same grid barriers, each graph stopping on its own. The initialisation
-// (masks, colours, first winner array, counters) is the kernel's first phase. Per graph the
-// rounds, the winners and the statistics are exactly those of kColorLoop.
+// Both colourings of a substep in ONE launch: the manifold graph (velocity solve) and the contact graph
+// (position solve), each the reference's Jones-Plassmann rounds: in a round every uncoloured entry whose
+// key is the largest at both ends takes the lowest colour free at both.
+//
+// An entry's colour and round depend only on the entries before it (larger key) at its two ends: with
+// each body's entries sorted by key and a body holding its first uncoloured one, an entry that is first at
+// both ends is coloured and both bodies move on. A round of the former loop cost two barriers and 64-bit
+// atomics on every remaining entry (8 to 13 us a round).
+//
+// Graphs of one cluster whose bodies fit a block's shared memory: one block a graph runs the rounds there,
+// two block barriers each (about 0.3 us a round). Larger ones: no rounds at all, every thread visits its
+// bodies and colours what is ready. The round of an entry is then one above the later of its
+// predecessors' rounds; entries beyond the round limit stay uncoloured, as in the rounds. A body's state is
+// one 128-bit word (first uncoloured entry + 1, its place in the lists, the body's colour mask) and a
+// 64-bit word (last round, the same place): each single-copy atomic, and taken together only when the
+// places agree, so no fences are needed. Only the thread that colours an entry writes its two bodies'
+// states.
 struct ColorJob {
   int ne, nb;          // entries, bodies
   int* col;            // [ne] colours out
-  long long *winA, *winB;
-  u64* mask;           // [nb]
-  int* aux;            // [0..2] remaining counts by round % 3, [3] max colour, [4] left uncoloured,
-                       // [5] rounds run
-  int *listA, *listB;  // [ne] each: every block's still-uncoloured entries, in its own chunk
-  int* blockCount;     // [gridDim] the blocks' list lengths, published for the tail
-  int *tailA, *tailB;  // [kColorTailMax] each: the tail's worklists (block 0 alone)
-  int tailAt;          // block 0 takes over once at most this many entries (both graphs) are left
-  int tailShared;      // the launch has the shared-memory tail's tables (dynamic shared memory)
+  u64* mask;           // [nb] colours of each body's entries out
+  int* aux;            // [0] list space taken, [2] largest round, [3] max colour, [4] left uncoloured, [5] rounds run
+  int *cnt, *at;       // [nb] entries of each body, their place in the lists
+  int4* list;          // [2 ne + nb] (key low, key high, entry, other body << 1 | 1 at its first end) unsorted
+  int2* sorted;        // [2 ne + nb] (entry, other body (or -1) << 1 | 1 at its first end), then (-1, 0)
+  uint4* state;        // [nb]
+  u64* round;          // [nb]
   // stable order by colour, built in the same launch when order is set: order[ne] (entry indices,
   // colour-major, index order within a colour), off[65] (first position of each colour key, then
   // ne), hist[64 * gridDim] (scratch)
   int *order = nullptr, *off = nullptr, *hist = nullptr;
 };
-// once at most ColorJob::tailAt entries (both colourings together) are left, block 0 alone runs the
-// remaining rounds with block barriers (in shared memory when they fit its tables), and the other
-// blocks wait at one grid barrier
-constexpr int kColorMaxChunks = 20;    // histogram row chunks of 32 blocks (grids up to 640 blocks)
-constexpr int kColorTailMax = 65536;  // largest tail hand-over the worklists are sized for
+constexpr size_t kColorMaxSmem = 200 * 1024;  // bodies of a graph in one block
+constexpr int kColorMaxChunks = 20;  // histogram row chunks of 32 blocks (grids up to 640 blocks)
 
 template <class R, bool MANIFOLD>
 __device__ __forceinline__ void colorInit(const Dev<R>& d, const ColorJob& J, long gtid, long gstride) {
   if (J.ne <= 0)
     return;  // a kept (or empty) graph: its colours and statistics stay as they are
-  for (long b = gtid; b < J.nb; b += gstride) {
-    J.mask[b] = 0ull;
-    J.winA[b] = -1ll;
-  }
+  for (long b = gtid; b < J.nb; b += gstride)
+    J.cnt[b] = 0;
   for (long i = gtid; i < J.ne; i += gstride) {
     if (MANIFOLD) {
       const int2 ab = d.mab[i];
@@ -365,78 +388,241 @@ __device__ __forceinline__ void colorInit(const Dev<R>& d, const ColorJob& J, lo
     J.aux[4] = 0;
   }
 }
-// Worklists. Block b owns the entries [b chunk, (b + 1) chunk). Round 0 walks them all (skipping
-// the coloured ones); every later round walks only the block's losers of the round before, kept
-// in its own segment of listA / listB (ping-pong) and counted in shared memory. A round's outcome
-// does not depend on the order its entries are visited in: the winners at one end are unique,
-// winners never share an end, and losers only reset the next round's slots.
-struct ColorRange {
-  const int* list;  // nullptr: round 0, the whole chunk
-  long first, count;
-};
-__device__ __forceinline__ ColorRange colorRange(const ColorJob& J, int round, int inCount) {
-  const long chunk = (J.ne + gridDim.x - 1) / gridDim.x;
-  const long first = (long)blockIdx.x * chunk;
-  if (round == 0) {
-    const long last = first + chunk < J.ne ? first + chunk : J.ne;
-    return ColorRange{nullptr, first, last > first ? last - first : 0};
-  }
-  return ColorRange{((round & 1) ? J.listB : J.listA) + first, first, inCount};
+// an entry's ends; an entry of one body (a wall's, or a body and its own image) has no second
+template <class R, bool MANIFOLD>
+__device__ __forceinline__ void colorTwoEnds(const Dev<R>& d, int i, int& ea, int& eb) {
+  colorEnds<R, MANIFOLD>(d, i, ea, eb);
+  if (eb == ea)
+    eb = -1;
 }
 template <class R, bool MANIFOLD>
-__device__ __forceinline__ void colorContend(const Dev<R>& d, const ColorJob& J, int round, const ColorRange& rg) {
-  long long* win = (round & 1) ? J.winB : J.winA;
-  if ((blockIdx.x | threadIdx.x) == 0)
-    J.aux[(round + 1) % 3] = 0;
-  for (long t = threadIdx.x; t < rg.count; t += blockDim.x) {
-    const long i = rg.list ? rg.list[t] : rg.first + t;
-    if (!rg.list && J.col[i] != -1)
-      continue;
-    int ea, eb;
-    colorEnds<R, MANIFOLD>(d, (int)i, ea, eb);
-    const long long k = entryKey<R, MANIFOLD>(d, (int)i, ea);
-    atomicMax(&win[ea], k);
-    if (eb >= 0)
-      atomicMax(&win[eb], k);
-  }
-}
-// losers go to the block's next list (shared-memory counter *outCount); the grid's loser count
-// for the round's stop test is added once per block by the caller
-template <class R, bool MANIFOLD>
-__device__ __forceinline__ void colorCommitTo(const Dev<R>& d, const ColorJob& J, int round, const ColorRange& rg,
-                                              int* out, int* outCount) {
-  long long* win = (round & 1) ? J.winB : J.winA;
-  long long* nxt = (round & 1) ? J.winA : J.winB;
-  for (long t = threadIdx.x; t < rg.count; t += blockDim.x) {
-    const long i = rg.list ? rg.list[t] : rg.first + t;
-    if (!rg.list && J.col[i] != -1)
-      continue;
-    int ea, eb;
-    colorEnds<R, MANIFOLD>(d, (int)i, ea, eb);
-    const long long k = entryKey<R, MANIFOLD>(d, (int)i, ea);
-    if (__ldcg(&win[ea]) != k || (eb >= 0 && __ldcg(&win[eb]) != k)) {
-      out[atomicAdd(outCount, 1)] = (int)i;
-      nxt[ea] = -1;
+__device__ __forceinline__ void colorCount(const Dev<R>& d, const ColorJob& J, long gtid, long gstride) {
+  for (long i = gtid; i < J.ne; i += gstride)
+    if (J.col[i] == -1) {
+      int ea, eb;
+      colorTwoEnds<R, MANIFOLD>(d, (int)i, ea, eb);
+      atomicAdd(&J.cnt[ea], 1);
       if (eb >= 0)
-        nxt[eb] = -1;
-      continue;
+        atomicAdd(&J.cnt[eb], 1);
     }
-    u64 forb = __ldcg(&J.mask[ea]);
-    if (eb >= 0)
-      forb |= __ldcg(&J.mask[eb]);
-    int cc = 0;
-    while (cc < 62 && (forb & (1ull << cc)))
-      ++cc;
-    J.col[i] = cc;
-    J.mask[ea] |= 1ull << cc;
-    if (eb >= 0)
-      J.mask[eb] |= 1ull << cc;
+}
+// room in the lists for every body, in any order
+__device__ __forceinline__ void colorRoom(const ColorJob& J, long gtid, long gstride) {
+  if (J.ne <= 0)
+    return;
+  const int lane = threadIdx.x & 31;
+  for (long b0 = gtid - lane; b0 < J.nb; b0 += gstride) {
+    const long b = b0 + lane;
+    const int n = b < J.nb ? __ldcg(&J.cnt[b]) : 0;
+    const int want = b < J.nb ? n + 1 : 0;  // and the end mark
+    int x = want;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o)
+        x += y;
+    }
+    int base = 0;
+    if (lane == 31)
+      base = atomicAdd(&J.aux[0], x);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (b < J.nb) {
+      J.at[b] = base + x - want;
+      J.cnt[b] = 0;  // now the entries filled in
+    }
   }
 }
 template <class R, bool MANIFOLD>
-__device__ __forceinline__ void colorCommit(const Dev<R>& d, const ColorJob& J, int round, const ColorRange& rg,
-                                            int* outCount) {
-  colorCommitTo<R, MANIFOLD>(d, J, round, rg, (((round + 1) & 1) ? J.listB : J.listA) + rg.first, outCount);
+__device__ __forceinline__ void colorFill(const Dev<R>& d, const ColorJob& J, long gtid, long gstride) {
+  for (long i = gtid; i < J.ne; i += gstride)
+    if (J.col[i] == -1) {
+      int ea, eb;
+      colorTwoEnds<R, MANIFOLD>(d, (int)i, ea, eb);
+      const long long k = entryKey<R, MANIFOLD>(d, (int)i, ea);
+      const int lo = (int)(k & 0xffffffffll), hi = (int)(k >> 32);
+      const int pa = __ldcg(&J.at[ea]) + atomicAdd(&J.cnt[ea], 1);
+      J.list[pa] = make_int4(lo, hi, (int)i, (eb << 1) | 1);
+      if (eb >= 0) {
+        const int pb = __ldcg(&J.at[eb]) + atomicAdd(&J.cnt[eb], 1);
+        J.list[pb] = make_int4(lo, hi, (int)i, ea << 1);
+      }
+    }
+}
+// each body's list by decreasing key, eight lanes a body: an element's place is the number of larger keys
+constexpr int kColorLanes = 8;
+__device__ __forceinline__ void colorSort(const ColorJob& J, long gtid, long gstride) {
+  if (J.ne <= 0)
+    return;
+  const int sub = threadIdx.x % kColorLanes;
+  for (long b = gtid / kColorLanes; b < J.nb; b += gstride / kColorLanes) {
+    const int n = __ldcg(&J.cnt[b]), at = __ldcg(&J.at[b]);
+    for (int k = sub; k < n; k += kColorLanes) {
+      const int4 e = __ldcg(&J.list[at + k]);
+      const u64 key = ((u64)(unsigned)e.y << 32) | (unsigned)e.x;
+      int rank = 0;
+      for (int q = 0; q < n; ++q) {
+        const int4 f = __ldcg(&J.list[at + q]);
+        rank += ((((u64)(unsigned)f.y << 32) | (unsigned)f.x) > key) ? 1 : 0;
+      }
+      J.sorted[at + rank] = make_int2(e.z, e.w);
+      if (rank == 0)
+        flowStoreGlobal(&J.state[b], (unsigned)e.z + 1u, (unsigned)at, 0u, 0u);
+    }
+    if (sub == 0) {
+      J.sorted[at + n] = make_int2(-1, 0);
+      J.round[b] = (u64)(unsigned)at;
+      if (n == 0)
+        flowStoreGlobal(&J.state[b], 0u, (unsigned)at, 0u, 0u);
+    }
+  }
+}
+// one visit of body b: colours its first entry if that is first at the other end too. Returns whether the
+// body has entries left.
+__device__ __forceinline__ bool colorVisit(const ColorJob& J, long b, int maxRounds, int& maxRound) {
+  for (;;) {
+    const uint4 s = flowLoadGlobal(&J.state[b]);
+    if (s.x == 0u) {
+      J.mask[b] = ((u64)s.w << 32) | s.z;
+      return false;
+    }
+    const int2 el = __ldcg(&J.sorted[s.y]);
+    if (!(el.y & 1))
+      return true;  // its first end's thread colours it
+    const int o = el.y >> 1;
+    const volatile u64* vr = J.round;
+    const u64 ra = vr[b];
+    if ((unsigned)ra != s.y)
+      return true;
+    uint4 t = make_uint4(0u, 0u, 0u, 0u);
+    u64 rb = 0ull;
+    if (o >= 0) {
+      t = flowLoadGlobal(&J.state[o]);
+      rb = vr[o];
+      if (t.x != s.x || (unsigned)rb != t.y)
+        return true;
+    }
+    const u64 ma = ((u64)s.w << 32) | s.z, mb = ((u64)t.w << 32) | t.z;
+    const int r = 1 + max((int)(ra >> 32), (int)(rb >> 32));
+    u64 bit = 0ull;
+    if (r <= maxRounds) {
+      const u64 open = ~(ma | mb) & ((1ull << 62) - 1ull);
+      const int cc = open ? __ffsll((long long)open) - 1 : 62;
+      J.col[s.x - 1u] = cc;
+      bit = 1ull << cc;
+      maxRound = max(maxRound, r);
+    }
+    auto advance = [&](long body, unsigned place, u64 m) {
+      const unsigned next = (unsigned)(__ldcg(&J.sorted[place + 1u]).x + 1);
+      *reinterpret_cast<volatile u64*>(&J.round[body]) = ((u64)(unsigned)r << 32) | (place + 1u);
+      flowStoreGlobal(&J.state[body], next, place + 1u, (unsigned)m, (unsigned)(m >> 32));
+    };
+    advance(b, s.y, ma | bit);
+    if (o >= 0)
+      advance(o, t.y, mb | bit);
+  }
+}
+// the rounds of one graph in one block, its bodies in shared memory
+struct ColorBody {
+  u64 mask;
+  int entry, other;  // first uncoloured entry (-1: none), its other body << 1 | 1 at its first end
+  int2 next;         // the one after it
+  int place, moved;  // place of `next` in the lists; the entry was coloured this round
+};
+__device__ __forceinline__ void colorRounds(const ColorJob& J, int maxRounds, ColorBody* B) {
+  for (int b = threadIdx.x; b < J.nb; b += blockDim.x) {
+    const int at = __ldcg(&J.at[b]);
+    const int2 el = __ldcg(&J.sorted[at]);
+    ColorBody c;
+    c.mask = 0ull;
+    c.entry = el.x;
+    c.other = el.y;
+    c.next = el.x >= 0 ? __ldcg(&J.sorted[at + 1]) : make_int2(-1, 0);
+    c.place = at + 1;
+    c.moved = 0;
+    B[b] = c;
+  }
+  __syncthreads();
+  int round = 0;
+  for (; round < maxRounds; ++round) {
+    int left = 0;
+    for (int b = threadIdx.x; b < J.nb; b += blockDim.x) {
+      const int e = B[b].entry;
+      if (e < 0)
+        continue;
+      left = 1;
+      const int ot = B[b].other, o = ot >> 1;
+      if (!(ot & 1) || (o >= 0 && B[o].entry != e))
+        continue;
+      const u64 ma = B[b].mask, mb = o >= 0 ? B[o].mask : 0ull;
+      const u64 open = ~(ma | mb) & ((1ull << 62) - 1ull);
+      const int cc = open ? __ffsll((long long)open) - 1 : 62;
+      J.col[e] = cc;
+      B[b].mask = ma | 1ull << cc;
+      B[b].moved = 1;
+      if (o >= 0) {
+        B[o].mask = mb | 1ull << cc;
+        B[o].moved = 1;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's bodies' next entries
+    if (!__syncthreads_or(left))
+      break;
+    for (int b = threadIdx.x; b < J.nb; b += blockDim.x)
+      if (B[b].moved) {
+        const int2 n = B[b].next;
+        B[b].entry = n.x;
+        B[b].other = n.y;
+        B[b].moved = 0;
+        if (n.x >= 0) {  // the end mark is the last
+          B[b].place += 1;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(&B[b].next)),
+                       "l"(J.sorted + B[b].place)
+                       : "memory");
+        }
+      }
+    __syncthreads();
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  for (int b = threadIdx.x; b < J.nb; b += blockDim.x)
+    J.mask[b] = B[b].mask;
+  if (threadIdx.x == 0)
+    J.aux[2] = round;
+}
+// all entries, in any order the states allow; false on time-out
+__device__ __forceinline__ bool colorRun(const ColorJob& jm, const ColorJob& jc, int maxRounds, const GridBar& gb, long gtid,
+                                         long gstride) {
+  int mr[2] = {0, 0};
+  long spins = 0;
+  bool late = false;
+  u64 open[2] = {~0ull, ~0ull};  // of the thread's first 64 bodies of a graph: those with entries left
+  for (bool more = true; more && !late;) {
+    more = false;
+    for (int g = 0; g < 2; ++g) {
+      const ColorJob& J = g ? jc : jm;
+      if (J.ne <= 0)
+        continue;
+      int k = 0;
+      for (long b = gtid; b < J.nb; b += gstride, ++k) {
+        if (k < 64 && !(open[g] >> k & 1ull))
+          continue;
+        if (colorVisit(J, b, maxRounds, mr[g]))
+          more = true;
+        else if (k < 64)
+          open[g] &= ~(1ull << k);
+      }
+    }
+    late = ++spins > gb.spins;
+  }
+  if (late)
+    atomicOr(gb.err, kErrBarrier);
+  const int m = __reduce_max_sync(__activemask(), max(mr[0], mr[1]));
+  if (m > 0 && (mr[0] == m || mr[1] == m)) {
+    if (jm.ne > 0)
+      atomicMax(&jm.aux[2], m);
+    if (jc.ne > 0)
+      atomicMax(&jc.aux[2], m);
+  }
+  return !late;
 }
 // ---- stable order by colour (counting sort over 64 keys: colours 0..62, 63 for uncoloured, the
 // order of the reference's stable sort by colour). Block b owns the contiguous chunk
@@ -572,7 +758,7 @@ __device__ __forceinline__ void colorOrderScatter(const ColorJob& J) {
 __device__ __forceinline__ void colorStats(const ColorJob& J, long gtid, long gstride) {
   int mxc = INT_MIN, left = 0;
   for (long i = gtid; i < J.ne; i += gstride) {
-    const int v = J.col[i];
+    const int v = __ldcg(&J.col[i]);
     mxc = v > mxc ? v : mxc;
     left += (v == -1) ? 1 : 0;
   }
@@ -590,226 +776,6 @@ __device__ __forceinline__ void colorStats(const ColorJob& J, long gtid, long gs
   }
 }
 
-// The tail, in block 0 alone: gather every block's remaining entries into one list, then run the
-// remaining rounds as the grid does (same contend / commit / stop rule), with block barriers.
-// Global writes of one round are seen by the next through the barrier (and the L2 reads of win and
-// mask in colorCommit).
-template <class R, bool MANIFOLD>
-__device__ __forceinline__ int colorTailGather(const ColorJob& J, int round, int* dst) {
-  // thread b copies block b's list to its offset (an exclusive scan of the list lengths; the
-  // grid has at most blockDim blocks)
-  __shared__ int sWarp[kColorBlock / 32];
-  __shared__ int sTotal;
-  const long chunk = (J.ne + gridDim.x - 1) / gridDim.x;
-  const int* src = (round & 1) ? J.listB : J.listA;  // the lists this round reads
-  const int b = threadIdx.x, lane = b & 31, w = b >> 5;
-  const int n = b < (int)gridDim.x ? J.blockCount[b] : 0;
-  int incl = n;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o)
-      incl += u;
-  }
-  if (lane == 31)
-    sWarp[w] = incl;
-  __syncthreads();
-  if (b == 0) {
-    int run = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-      const int c = sWarp[q];
-      sWarp[q] = run;
-      run += c;
-    }
-    sTotal = run;
-  }
-  __syncthreads();
-  const int off = sWarp[w] + incl - n;
-  for (int t = 0; t < n; ++t)
-    dst[off + t] = src[(long)b * chunk + t];
-  __threadfence_block();
-  __syncthreads();
-  return sTotal;
-}
-template <class R>
-__device__ void colorTail(const Dev<R>& d, const ColorJob& jm, const ColorJob& jc, int round, int maxRounds,
-                          bool doneM, bool doneC, int prevM, int prevC) {
-  __shared__ int sOut[2];
-  int nM = doneM ? 0 : colorTailGather<R, true>(jm, round, jm.tailA);
-  int nC = doneC ? 0 : colorTailGather<R, false>(jc, round, jc.tailA);
-  for (int k = 0; round < maxRounds && !(doneM && doneC); ++round, ++k) {
-    const int* inM = (k & 1) ? jm.tailB : jm.tailA;
-    const int* inC = (k & 1) ? jc.tailB : jc.tailA;
-    int* outM = (k & 1) ? jm.tailA : jm.tailB;
-    int* outC = (k & 1) ? jc.tailA : jc.tailB;
-    if (threadIdx.x == 0)
-      sOut[0] = sOut[1] = 0;
-    const ColorRange rm{inM, 0, nM}, rc{inC, 0, nC};
-    if (!doneM)
-      colorContend<R, true>(d, jm, round, rm);
-    if (!doneC)
-      colorContend<R, false>(d, jc, round, rc);
-    __syncthreads();  // block 0 alone: the block barrier orders its global accesses
-    if (!doneM)
-      colorCommitTo<R, true>(d, jm, round, rm, outM, &sOut[0]);
-    if (!doneC)
-      colorCommitTo<R, false>(d, jc, round, rc, outC, &sOut[1]);
-    __syncthreads();  // block 0 alone: the block barrier orders its global accesses
-    const int remM = sOut[0], remC = sOut[1];
-    if (threadIdx.x == 0) {
-      if (!doneM)
-        jm.aux[round % 3] = remM;
-      if (!doneC)
-        jc.aux[round % 3] = remC;
-    }
-    if (!doneM) {
-      doneM = remM == 0 || remM == prevM;
-      prevM = remM;
-      nM = remM;
-    }
-    if (!doneC) {
-      doneC = remC == 0 || remC == prevC;
-      prevC = remC;
-      nC = remC;
-    }
-    __syncthreads();
-  }
-}
-
-// The tail in shared memory (block 0 alone, at most kTailShEntries entries of both graphs): every
-// body the remaining entries touch gets a slot of a hash table (code body * 2 + graph), holding its
-// winner word and colour mask, so a round touches no global memory but the final colours. The
-// rounds, winners and colours are those of colorTail: contend (max of the keys at both ends), win
-// with the maximum at both ends, take the lowest colour free at both ends; the losers contend
-// again. One winner word per slot suffices: after each commit the words of every end touched that
-// round go back to -1, and the next round's contenders are that round's losers.
-constexpr int kTailShEntries = 1024;
-constexpr int kTailShSlots = 4096;  // a power of two, at least 2 ends x entries x 2
-struct TailShared {
-  u64 mask[kTailShSlots];
-  long long win[kTailShSlots];
-  long long key[kTailShEntries];
-  int body[kTailShSlots];  // code of the slot's body, -1 free
-  int ent[kTailShEntries];
-  short la[kTailShEntries], lb[kTailShEntries];  // slots of the ends (lb -1: no second body)
-  short list[2][kTailShEntries];                 // entries of this round and the next
-  unsigned char g[kTailShEntries];               // 0 manifold graph, 1 contact graph
-};
-__device__ __forceinline__ int tailSlot(TailShared& S, int code) {
-  const unsigned h = (unsigned)code * 2654435761u;
-  for (int probe = 0; probe < kTailShSlots; ++probe) {  // at most 2 x kTailShEntries codes: a slot is free
-    const int s = (int)((h + (unsigned)probe) & (kTailShSlots - 1));
-    const int prev = atomicCAS(&S.body[s], -1, code);
-    if (prev == -1 || prev == code)
-      return s;
-  }
-  return 0;
-}
-template <class R, bool MANIFOLD>
-__device__ __forceinline__ void tailEntry(const Dev<R>& d, TailShared& S, int t, int i, int g) {
-  int ea, eb;
-  colorEnds<R, MANIFOLD>(d, i, ea, eb);
-  S.ent[t] = i;
-  S.g[t] = (unsigned char)g;
-  S.key[t] = entryKey<R, MANIFOLD>(d, i, ea);
-  S.la[t] = (short)tailSlot(S, 2 * ea + g);
-  S.lb[t] = (short)(eb >= 0 ? tailSlot(S, 2 * eb + g) : -1);
-  S.list[0][t] = (short)t;
-}
-template <class R>
-__device__ void colorTailShared(const Dev<R>& d, const ColorJob& jm, const ColorJob& jc, int round, int maxRounds,
-                                bool doneM, bool doneC, int prevM, int prevC) {
-  extern __shared__ __align__(16) unsigned char tailSmem[];
-  TailShared& S = *reinterpret_cast<TailShared*>(tailSmem);
-  __shared__ int sLose[2], sNext;
-  const int nM = doneM ? 0 : colorTailGather<R, true>(jm, round, jm.tailA);
-  const int nC = doneC ? 0 : colorTailGather<R, false>(jc, round, jc.tailA);
-  for (int s = threadIdx.x; s < kTailShSlots; s += blockDim.x)
-    S.body[s] = -1;
-  __syncthreads();
-  for (int t = threadIdx.x; t < nM + nC; t += blockDim.x) {
-    if (t < nM)
-      tailEntry<R, true>(d, S, t, jm.tailA[t], 0);
-    else
-      tailEntry<R, false>(d, S, t, jc.tailA[t - nM], 1);
-  }
-  __syncthreads();
-  for (int s = threadIdx.x; s < kTailShSlots; s += blockDim.x) {
-    const int code = S.body[s];
-    if (code >= 0)
-      S.mask[s] = __ldcg(&((code & 1) ? jc.mask : jm.mask)[code >> 1]);
-    S.win[s] = -1;
-  }
-  int cnt = nM + nC;
-  for (int k = 0; round < maxRounds && !(doneM && doneC); ++round, ++k) {
-    const short* in = S.list[k & 1];
-    short* out = S.list[(k + 1) & 1];
-    if (threadIdx.x == 0)
-      sLose[0] = sLose[1] = sNext = 0;
-    __syncthreads();  // the slots' words and masks, and the counters, are set
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      const int t = in[j];
-      if (S.g[t] ? doneC : doneM)
-        continue;
-      atomicMax(&S.win[S.la[t]], S.key[t]);
-      if (S.lb[t] >= 0)
-        atomicMax(&S.win[S.lb[t]], S.key[t]);
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      const int t = in[j];
-      const int g = S.g[t];
-      if (g ? doneC : doneM)
-        continue;
-      const int la = S.la[t], lb = S.lb[t];
-      const long long key = S.key[t];
-      if (S.win[la] != key || (lb >= 0 && S.win[lb] != key)) {
-        out[atomicAdd(&sNext, 1)] = (short)t;
-        atomicAdd(&sLose[g], 1);
-        continue;
-      }
-      const u64 forb = S.mask[la] | (lb >= 0 ? S.mask[lb] : 0ull);
-      int cc = 0;
-      while (cc < 62 && (forb & (1ull << cc)))
-        ++cc;
-      (g ? jc : jm).col[S.ent[t]] = cc;
-      S.mask[la] |= 1ull << cc;  // the round's winners share no end
-      if (lb >= 0)
-        S.mask[lb] |= 1ull << cc;
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-      const int t = in[j];
-      if (S.g[t] ? doneC : doneM)
-        continue;
-      S.win[S.la[t]] = -1;
-      if (S.lb[t] >= 0)
-        S.win[S.lb[t]] = -1;
-    }
-    const int remM = sLose[0], remC = sLose[1];
-    cnt = sNext;
-    if (threadIdx.x == 0) {
-      if (!doneM)
-        jm.aux[round % 3] = remM;
-      if (!doneC)
-        jc.aux[round % 3] = remC;
-    }
-    if (!doneM) {
-      doneM = remM == 0 || remM == prevM;
-      prevM = remM;
-    }
-    if (!doneC) {
-      doneC = remC == 0 || remC == prevC;
-      prevC = remC;
-    }
-    __syncthreads();  // the counters are read before the next round resets them
-  }
-  for (int s = threadIdx.x; s < kTailShSlots; s += blockDim.x) {  // the bodies' colour masks
-    const int code = S.body[s];
-    if (code >= 0)
-      ((code & 1) ? jc.mask : jm.mask)[code >> 1] = S.mask[s];
-  }
-}
-
 // job 0: manifolds over real bodies (skipped when ne = 0), job 1: contacts over body slots.
 // CLUSTER: the launch is one thread-block cluster (graphs of a few tens of thousands of entries)
 // and the hardware cluster barrier replaces the grid-wide one, as in kSweepLoop.
@@ -817,8 +783,7 @@ __device__ void colorTailShared(const Dev<R>& d, const ColorJob& jm, const Color
 // contact list changed, differ[1]: the manifold list changed; reuse = 0 forces both colourings)
 template <class R, bool CLUSTER = false>
 __global__ void __launch_bounds__(kColorBlock) kColorBoth(Dev<R> d, ColorJob jm, ColorJob jc, int maxRounds,
-                                                          GridBar gb, const int* differ, int reuse) {
-  __shared__ int sCount[2][2];  // per job: this block's loser counts, ping-pong by round
+                                                          GridBar gb, const int* differ, int reuse, int inShared) {
   const long gtid = (long)blockIdx.x * blockDim.x + threadIdx.x, gstride = (long)gridDim.x * blockDim.x;
   if (reuse && !differ[1])
     jm.ne = 0;  // uniform over the grid: the flags are written before the launch
@@ -828,76 +793,39 @@ __global__ void __launch_bounds__(kColorBlock) kColorBoth(Dev<R> d, ColorJob jm,
     return;
   colorInit<R, true>(d, jm, gtid, gstride);
   colorInit<R, false>(d, jc, gtid, gstride);
-  if (threadIdx.x < 4)
-    sCount[threadIdx.x >> 1][threadIdx.x & 1] = 0;
   if (!loopBarrier<CLUSTER>(gb))
     return;
-  int prevM = -1, prevC = -1;
-  bool doneM = jm.ne <= 0, doneC = jc.ne <= 0;
-  int round = 0;
-  bool tail = false;
-  for (; round < maxRounds && !(doneM && doneC); ++round) {
-    const int in = round & 1, outS = in ^ 1;  // shared counter slots: this round's list, the next
-    const ColorRange rm = colorRange(jm, round, sCount[0][in]), rc = colorRange(jc, round, sCount[1][in]);
-    if (!doneM)
-      colorContend<R, true>(d, jm, round, rm);
-    if (!doneC)
-      colorContend<R, false>(d, jc, round, rc);
-    if (!loopBarrier<CLUSTER>(gb))
-      return;
-    if (!doneM)
-      colorCommit<R, true>(d, jm, round, rm, &sCount[0][outS]);
-    if (!doneC)
-      colorCommit<R, false>(d, jc, round, rc, &sCount[1][outS]);
-    __syncthreads();
-    if (threadIdx.x == 0) {  // this block's losers into the grid's count; its consumed slot reset
-      if (!doneM && sCount[0][outS])
-        atomicAdd(&jm.aux[round % 3], sCount[0][outS]);
-      if (!doneC && sCount[1][outS])
-        atomicAdd(&jc.aux[round % 3], sCount[1][outS]);
-      sCount[0][in] = sCount[1][in] = 0;
-    }
-    if (!loopBarrier<CLUSTER>(gb))
-      return;
-    if (!doneM) {
-      const int rem = *reinterpret_cast<volatile int*>(&jm.aux[round % 3]);
-      doneM = rem == 0 || rem == prevM;
-      prevM = rem;
-    }
-    if (!doneC) {
-      const int rem = *reinterpret_cast<volatile int*>(&jc.aux[round % 3]);
-      doneC = rem == 0 || rem == prevC;
-      prevC = rem;
-    }
-    // few entries left: publish this block's lists, and block 0 takes over (uniform decision)
-    if (!(doneM && doneC) && round + 1 < maxRounds && gridDim.x <= blockDim.x &&
-        (doneM ? 0 : prevM) + (doneC ? 0 : prevC) <= jm.tailAt) {
-      if (threadIdx.x == 0) {
-        jm.blockCount[blockIdx.x] = doneM ? 0 : sCount[0][(round + 1) & 1];
-        jc.blockCount[blockIdx.x] = doneC ? 0 : sCount[1][(round + 1) & 1];
-      }
-      tail = true;
-      ++round;
-      break;
-    }
+  colorCount<R, true>(d, jm, gtid, gstride);
+  colorCount<R, false>(d, jc, gtid, gstride);
+  if (!loopBarrier<CLUSTER>(gb))
+    return;
+  colorRoom(jm, gtid, gstride);
+  colorRoom(jc, gtid, gstride);
+  if (!loopBarrier<CLUSTER>(gb))
+    return;
+  colorFill<R, true>(d, jm, gtid, gstride);
+  colorFill<R, false>(d, jc, gtid, gstride);
+  if (!loopBarrier<CLUSTER>(gb))
+    return;
+  colorSort(jm, gtid, gstride);
+  colorSort(jc, gtid, gstride);
+  if (!loopBarrier<CLUSTER>(gb))
+    return;
+  if (CLUSTER && inShared) {
+    extern __shared__ __align__(16) unsigned char colorSmem[];
+    if (blockIdx.x < 2 && (blockIdx.x ? jc.ne : jm.ne) > 0)
+      colorRounds(blockIdx.x ? jc : jm, maxRounds, reinterpret_cast<ColorBody*>(colorSmem));
+  } else {
+    colorRun(jm, jc, maxRounds, gb, gtid, gstride);
   }
-  if (tail) {
-    if (!loopBarrier<CLUSTER>(gb))  // the published lists are complete
-      return;
-    if (blockIdx.x == 0) {
-      if (jm.tailShared)
-        colorTailShared(d, jm, jc, round, maxRounds, doneM, doneC, prevM, prevC);
-      else
-        colorTail(d, jm, jc, round, maxRounds, doneM, doneC, prevM, prevC);
-    }
-    if (!loopBarrier<CLUSTER>(gb))  // the tail's colours are visible to every block
-      return;
-  }
+  if (!loopBarrier<CLUSTER>(gb))  // every colour is visible
+    return;
   if (gtid == 0) {
+    const int rounds = max(jm.ne > 0 ? __ldcg(&jm.aux[2]) : 0, jc.ne > 0 ? __ldcg(&jc.aux[2]) : 0);
     if (jm.ne > 0)
-      jm.aux[5] = round;
+      jm.aux[5] = rounds;
     if (jc.ne > 0)
-      jc.aux[5] = round;
+      jc.aux[5] = rounds;
   }
   colorStats(jm, gtid, gstride);
   colorStats(jc, gtid, gstride);

@@ -95,7 +95,6 @@ void Sim<R>::allocate(int cap, int mp, int mc) {
     b->ensure(cap, false, stream_);
   grounded_.ensure(cap, false, stream_);
   matId_.ensure(cap, false, stream_);
-  winner_.ensure(cap, false, stream_);
   mask_.ensure(cap, false, stream_);
   pairs_.ensure(mp, false, stream_);
   allocContactBuffers(mc);
@@ -143,7 +142,6 @@ void Sim<R>::ensureCapacity(int nc) {
     b->ensure(nc, true, stream_);
   grounded_.ensure(nc, true, stream_);
   matId_.ensure(nc, true, stream_);
-  winner_.ensure(nc, true, stream_);
   mask_.ensure(nc, true, stream_);
   capacity_ = nc;
   refreshDev();
@@ -187,7 +185,7 @@ void Sim<R>::refreshDev() {
   d.invMass = invMass_.p, d.scale = scale_.p, d.targetScale = target_.p, d.rad = rad_.p;
   d.planeFric = planeFric_.p;
   d.shapeId = shapeId_.p, d.realIdx = realIdx_.p, d.counts = counts_.p;
-  d.grounded = grounded_.p, d.matId = matId_.p, d.winner = winner_.p, d.mask = mask_.p;
+  d.grounded = grounded_.p, d.matId = matId_.p, d.mask = mask_.p;
   d.pairs = pairs_.p;
   d.cab = cab_.p, d.cn = cn_.p, d.crA = crA_.p, d.crB = crB_.p, d.cbv = cbv_.p;
   d.cColor = cColor_.p, d.cSlot = cSlot_.p, d.posLamC = posLamC_.p;
@@ -233,6 +231,7 @@ void Sim<R>::readBack(void* host, const void* dev, size_t bytes) {
 template <class R>
 void Sim<R>::clearLoopError() {
   dropPending();
+  topoValid_ = false;  // the loops' products are partial
   cudaCheck(cudaMemsetAsync(&ctr_.p->err, 0, sizeof(int), stream_), "memset error bits");
   sync();
 }
@@ -283,33 +282,12 @@ void Sim<R>::launchCoop(K kernel, A... args) {
 }
 template <class R>
 template <class K, class... A>
-void Sim<R>::launchCoopSmem(K kernel, int block, size_t smem, A... args) {
-  const auto key = std::make_tuple(reinterpret_cast<const void*>(kernel), block, smem);
-  auto it = coopPerSmem_.find(key);
-  if (it == coopPerSmem_.end()) {
-    cudaCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
-    int per = 0;
-    cudaCheck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, smem), "occupancy");
-    if (per < 1)
-      throw CudaError("persistent loop kernel cannot be resident");
-    it = coopPerSmem_.emplace(key, per).first;
-  }
-  gbar_.ensure(2, false, stream_);
-  cudaCheck(cudaMemsetAsync(gbar_.p, 0, 2 * sizeof(unsigned), stream_), "memset barrier");
-  void* argv[] = {static_cast<void*>(&args)...};
-  ++launches_;
-  cudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(std::min(it->second, 4) * numSMs_),
-                                        dim3(block), argv, smem, stream_),
-            "cooperative launch");
-}
-template <class R>
-template <class K, class... A>
 bool Sim<R>::launchCluster(K kernel, A... args) {
-  return launchClusterCfg(kernel, sweepClusterBlocks_, kBlock, 0, args...);
+  return launchClusterCfg(kernel, sweepClusterBlocks_, kBlock, 0, 0, args...);
 }
 template <class R>
 template <class K, class... A>
-bool Sim<R>::launchClusterCfg(K kernel, int blocks, int block, size_t smem, A... args) {
+bool Sim<R>::launchClusterCfg(K kernel, int blocks, int block, size_t smem, size_t maxSmem, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(block);
@@ -328,12 +306,14 @@ bool Sim<R>::launchClusterCfg(K kernel, int blocks, int block, size_t smem, A...
     int clusters = 0;
     if (blocks > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
       (void)cudaGetLastError();
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (maxSmem > 48 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem) != cudaSuccess)
       (void)cudaGetLastError();
+    cfg.dynamicSmemBytes = maxSmem;
     if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess)
       (void)cudaGetLastError();
     it = clusterOk_.emplace(key, clusters >= 1 ? 1 : 0).first;
+    cfg.dynamicSmemBytes = smem;
   }
   if (!it->second)
     return false;
@@ -1492,22 +1472,19 @@ void Sim<R>::colorBoth(int nm, int nc, int& ncolV, int& velLeft, int& ncolP, int
     return;
   mask_.ensure(std::max(nbM, 1), false, stream_);
   maskP_.ensure(std::max(nbC, 1), false, stream_);
-  winner_.ensure(std::max(nbM, 1), false, stream_);
-  winner2_.ensure(std::max(nbM, 1), false, stream_);
-  winnerP_.ensure(std::max(nbC, 1), false, stream_);
-  winnerP2_.ensure(std::max(nbC, 1), false, stream_);
   colorAux_.ensure(12, false, stream_);
-  colorListM_.ensure(2 * std::max(neM, 1), false, stream_);
-  colorListC_.ensure(2 * std::max(neC, 1), false, stream_);
-  // per job: the blocks' list lengths (up to 4 blocks per SM), then the tail's two lists
+  auto job = [&](int ne, int nb, int* col, u64* mask, int* aux, ColorBuf& f) {
+    const size_t n1 = (size_t)std::max(nb, 1), n2 = 2 * (size_t)std::max(ne, 1) + n1;
+    f.cnt.ensure(2 * n1, false, stream_);
+    f.list.ensure(n2, false, stream_);
+    f.sorted.ensure(n2, false, stream_);
+    f.state.ensure(n1, false, stream_);
+    f.round.ensure(n1, false, stream_);
+    return ColorJob{ne, nb, col, mask, aux, f.cnt.p, f.cnt.p + n1, f.list.p, f.sorted.p, f.state.p, f.round.p};
+  };
   const int maxGrid = 4 * numSMs_;
-  colorTail_.ensure(2 * (maxGrid + 2 * (size_t)kColorTailMax), false, stream_);
-  int* tm = colorTail_.p;
-  int* tc = colorTail_.p + maxGrid + 2 * kColorTailMax;
-  ColorJob jm{neM, nbM, mColor_.p, winner_.p, winner2_.p, mask_.p, colorAux_.p, colorListM_.p,
-              colorListM_.p + std::max(neM, 1), tm, tm + maxGrid, tm + maxGrid + kColorTailMax, std::min(colorTailAt_, kColorTailMax)};
-  ColorJob jc{neC, nbC, cColor_.p, winnerP_.p, winnerP2_.p, maskP_.p, colorAux_.p + 6, colorListC_.p,
-              colorListC_.p + std::max(neC, 1), tc, tc + maxGrid, tc + maxGrid + kColorTailMax, std::min(colorTailAt_, kColorTailMax)};
+  ColorJob jm = job(neM, nbM, mColor_.p, mask_.p, colorAux_.p, colorM_);
+  ColorJob jc = job(neC, nbC, cColor_.p, maskP_.p, colorAux_.p + 6, colorC_);
   if (!batch_) {  // the colour orders come out of the same launch (the batched form orders by scene)
     colorHist_.ensure(2 * 64 * (size_t)maxGrid, false, stream_);
     if (neM > 0) {
@@ -1523,15 +1500,14 @@ void Sim<R>::colorBoth(int nm, int nc, int& ncolV, int& velLeft, int& ncolP, int
   }
   gbar_.ensure(2, false, stream_);
   const GridBar gb{gbar_.p, &ctr_.p->err, barrierSleepNs_, barrierSpins_};
-  // the tail in shared memory when the hand-over fits its tables
-  const bool tailShared = std::min(colorTailAt_, kColorTailMax) <= kTailShEntries;
-  jm.tailShared = jc.tailShared = tailShared ? 1 : 0;
-  const size_t tailSmem = tailShared ? sizeof(TailShared) : 0;
+  // the rounds of both graphs in one block each while their bodies fit its shared memory
+  const size_t bodySmem = (size_t)std::max(nbM, nbC) * sizeof(ColorBody);
+  const bool inShared = bodySmem <= kColorMaxSmem && sweepClusterBlocks_ >= 2;
   const bool inCluster =
       std::max(neM, neC) <= colorClusterEntries_ && colorBlock_ == kColorBlock &&
       (cudaMemsetAsync(gbar_.p, 0, 2 * sizeof(unsigned), stream_) == cudaSuccess) &&
-      launchClusterCfg(kColorBoth<R, true>, sweepClusterBlocks_, kColorBlock, tailSmem, d_, jm, jc,
-                       std::max(nbM, nbC) + 2, gb, (const int*)topoFlags_.p, topoValid_ ? 1 : 0);
+      launchClusterCfg(kColorBoth<R, true>, sweepClusterBlocks_, kColorBlock, inShared ? bodySmem : 0, kColorMaxSmem, d_, jm, jc,
+                       std::max(nbM, nbC) + 2, gb, (const int*)topoFlags_.p, topoValid_ ? 1 : 0, inShared ? 1 : 0);
   // batched form: the launch-shape autotuner's colouring candidates (see colorTuning_)
   const bool tuneColor = !inCluster && batch_ && colorTuning_;
   const int slot = colorTuneStep_ % (kColorTuneCands * kTuneRounds);
@@ -1544,8 +1520,8 @@ void Sim<R>::colorBoth(int nm, int nc, int& ncolV, int& velLeft, int& ncolP, int
     cudaCheck(cudaEventRecord(colorTuneEv_[slot][0], stream_), "event");
   }
   if (!inCluster)
-    launchCoopSmem(kColorBoth<R>, colorBlock_, tailSmem, d_, jm, jc, std::max(nbM, nbC) + 2, gb,
-                   (const int*)topoFlags_.p, topoValid_ ? 1 : 0);
+    launchCoopB(kColorBoth<R>, colorBlock_, d_, jm, jc, std::max(nbM, nbC) + 2, gb, (const int*)topoFlags_.p,
+                topoValid_ ? 1 : 0, 0);
   if (tuneColor) {
     cudaCheck(cudaEventRecord(colorTuneEv_[slot][1], stream_), "event");
     if (++colorTuneStep_ == kColorTuneCands * kTuneRounds) {

@@ -212,7 +212,6 @@ class Sim {
   DBuf<R> invMass_, scale_, target_, rad_, planeFric_;
   DBuf<int> shapeId_, realIdx_, counts_;
   DBuf<uint8_t> grounded_, matId_;
-  DBuf<long long> winner_;
   DBuf<u64> mask_;
   DBuf<int2> pairs_;
   DBuf<int2> cab_;
@@ -226,8 +225,15 @@ class Sim {
   DBuf<uint8_t> persistent_, sideFlags_;
   DBuf<int> heights_, ordChanged_, ordKeysIn_, ordKeys_, ordPermIn_, ordPerm_;  // "ordered" pass
   DBuf<R> sdfA_, sdfB_;  // get_sdf_grid ping-pong
-  DBuf<int> colorListM_, colorListC_;  // colouring worklists (two halves each)
-  DBuf<int> colorTail_;                // block list lengths and the tail's worklists
+  // per graph: the bodies' entry counts and places, lists and states of the colouring (ColorJob)
+  struct ColorBuf {
+    DBuf<int> cnt;
+    DBuf<int4> list;
+    DBuf<int2> sorted;
+    DBuf<uint4> state;
+    DBuf<u64> round;
+  };
+  ColorBuf colorM_, colorC_;
   DBuf<int> sdfState_;
   DBuf<R> lambda_, prevLambda_, vn0_, posImp_, prevPosImp_;
   DBuf<Q4<R>> lambdaT_, prevLambdaT_, vt0_;
@@ -290,10 +296,8 @@ class Sim {
   void batchBounds(int nm);
   void ctl(int op, R thr, int mode);
   DBuf<unsigned> gbar_;        // grid barrier of the persistent loops
-  DBuf<long long> winner2_;    // second winner array of the colouring rounds
-  DBuf<long long> winnerP_, winnerP2_;  // winner arrays of the contact colouring
   DBuf<u64> maskP_;                     // colour masks of the contact colouring
-  DBuf<int> colorAux_;         // colouring, per graph (5 each): remaining counts [3], statistics [2]
+  DBuf<int> colorAux_;         // colouring, per graph (6 each; ColorJob::aux)
   // scratch
   DBuf<char> cubTmp_;
   DBuf<int> iA_, iB_, iC_, iD_, iE_;
@@ -393,18 +397,15 @@ class Sim {
   void launchCoopB(K kernel, int block, A... args);
   template <class K, class... A>
   void launchCoop(K kernel, A... args);
-  // cooperative launch with `smem` bytes of dynamic shared memory (resident blocks counted with it)
-  template <class K, class... A>
-  void launchCoopSmem(K kernel, int block, size_t smem, A... args);
-  std::map<std::tuple<const void*, int, size_t>, int> coopPerSmem_;  // by (kernel, block, smem)
   // one thread-block cluster of sweepClusterBlocks_ blocks; false when such a cluster cannot be
   // resident
   template <class K, class... A>
   bool launchCluster(K kernel, A... args);
-  // one cluster of `blocks` blocks of `block` threads with `smem` bytes of dynamic shared memory;
-  // false (nothing launched) when such a cluster cannot be resident. Residency is cached per kernel.
+  // one cluster of `blocks` blocks of `block` threads with `smem` (at most maxSmem) bytes of dynamic
+  // shared memory; false (nothing launched) when such a cluster cannot be resident with maxSmem.
+  // Residency is cached per kernel.
   template <class K, class... A>
-  bool launchClusterCfg(K kernel, int blocks, int block, size_t smem, A... args);
+  bool launchClusterCfg(K kernel, int blocks, int block, size_t smem, size_t maxSmem, A... args);
   // largest colouring (entries of the larger graph) run in one cluster (PDEM_COLOR_CLUSTER_ENTRIES)
   long colorClusterEntries_ = [] {
     const char* e = std::getenv("PDEM_COLOR_CLUSTER_ENTRIES");
@@ -516,14 +517,6 @@ class Sim {
   int tunedColorBlock() const { return (batch_ && colorTuning_) ? 0 : colorBlock_; }
   const float* colorTuneMs() const { return colorTuneMs_; }
  private:
-  // entries left (both colourings) at which block 0 alone finishes the colouring; PDEM_COLOR_TAIL
-  // overrides it (0 .. kColorTailMax). Measured: 1024 and 4096 alike on the 262k-sphere step, 1024
-  // 6 % faster on the batched drums, 16384 and up far slower (one block, many entries a round)
-  int colorTailAt_ = [] {
-    const char* e = std::getenv("PDEM_COLOR_TAIL");
-    const long v = e ? std::strtol(e, nullptr, 10) : 1024;
-    return (int)std::max(0L, std::min(v, 1L << 30));  // capped at kColorTailMax where used
-  }();
   // back-off (ns) between polls of a waiting block at a grid barrier; PDEM_BARRIER_SLEEP_NS
   // overrides it
   // polls before a grid-barrier wait gives up (setBarrierSpins; <= 0 restores kBarrierSpins)
