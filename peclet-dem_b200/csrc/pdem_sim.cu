@@ -1604,10 +1604,8 @@ void Sim<R>::buildIncidence(int kind, int ne, int nb) {
     ++launches_, kIncidenceKeys<R, 0><<<gridFor(ne), kBlock, 0, stream_>>>(d_, ne, incKeys_.p, incVals_.p, nb);
   else if (kind == 1)
     ++launches_, kIncidenceKeys<R, 1><<<gridFor(ne), kBlock, 0, stream_>>>(d_, ne, incKeys_.p, incVals_.p, nb);
-  else if (kind == 2)
-    ++launches_, kIncidenceKeys<R, 2><<<gridFor(ne), kBlock, 0, stream_>>>(d_, ne, incKeys_.p, incVals_.p, nb);
   else
-    ++launches_, kIncidenceKeys<R, 3><<<gridFor(ne), kBlock, 0, stream_>>>(d_, ne, incKeys_.p, incVals_.p, nb);
+    ++launches_, kIncidenceKeys<R, 2><<<gridFor(ne), kBlock, 0, stream_>>>(d_, ne, incKeys_.p, incVals_.p, nb);
   KCHECK("incidence keys");
   sortPairs(incKeys_.p, incKeysS_.p, incVals_.p, incValsS_.p, n2, bitsFor(nb));
   ++launches_, kLowerBoundOffsets<int><<<gridFor(nb + 1), kBlock, 0, stream_>>>(n2, incKeysS_.p, nb, incOff_.p);
@@ -2234,12 +2232,11 @@ void Sim<R>::hertzCommitHistory() {
     hzPrevCount_ = 0;
     return;
   }
-  lpermIn_.ensure(n, false, stream_);
-  lperm_.ensure(n, false, stream_);
-  ++launches_, kIota<R><<<gridFor(n), kBlock, 0, stream_>>>(lpermIn_.p, n);
-  sortPairs(hzKeys_.p, hzPrevKeys_.p, lpermIn_.p, lperm_.p, n, 64);
-  ++launches_, kHertzGatherPrev<<<gridFor(n), kBlock, 0, stream_>>>(n, lperm_.p, hzXi_.p, hzPrevXi_.p);
-  KCHECK("hertz commit history");
+  // the list becomes the previous one as it stands (in pair order)
+  std::swap(hzKeys_.p, hzPrevKeys_.p);
+  std::swap(hzKeys_.n, hzPrevKeys_.n);
+  std::swap(hzXi_.p, hzPrevXi_.p);
+  std::swap(hzXi_.n, hzPrevXi_.n);
   hzPrevCount_ = n;
 }
 // src/sim.hpp:545-594
@@ -2248,25 +2245,12 @@ void Sim<R>::hertzRebuildPairs(R skin) {
   cudaCheck(cudaMemcpyAsync(posPred_.p, pos_.p, capacity_ * sizeof(Q4<R>), cudaMemcpyDeviceToDevice, stream_), "D2D");
   const int np = findCollisionsGrow(skin, posPred_.p);
   const size_t need = pairs_.n;
-  if (hzXi_.n < need) {
-    // fresh buffers, as the reference reallocates (the previous history was committed above)
-    DBuf<u64> pk;
-    DBuf<Q4<R>> px;
-    pk.ensure(need, false, stream_);
-    px.ensure(need, false, stream_);
-    if (hzPrevCount_ > 0) {
-      cudaCheck(cudaMemcpyAsync(pk.p, hzPrevKeys_.p, hzPrevCount_ * sizeof(u64), cudaMemcpyDeviceToDevice, stream_), "D2D");
-      cudaCheck(cudaMemcpyAsync(px.p, hzPrevXi_.p, hzPrevCount_ * sizeof(Q4<R>), cudaMemcpyDeviceToDevice, stream_), "D2D");
-    }
-    sync();
-    std::swap(pk.p, hzPrevKeys_.p);
-    std::swap(pk.n, hzPrevKeys_.n);
-    std::swap(px.p, hzPrevXi_.p);
-    std::swap(px.n, hzPrevXi_.n);
-    hzXi_.ensure(need, false, stream_);
-    hzSnPair_.ensure(need, false, stream_);
-    hzKeys_.ensure(need, false, stream_);
-  }
+  hzXi_.ensure(need, false, stream_);
+  hzSnPair_.ensure(need, false, stream_);
+  hzKeys_.ensure(need, false, stream_);
+  hzOn_.ensure(need / 32 + 1, false, stream_);
+  hzNext_.ensure(2 * need, false, stream_);
+  cudaCheck(cudaMemsetAsync(hzOn_.p, 0xff, (np / 32 + 1) * sizeof(unsigned), stream_), "memset");
   if (np > 0) {
     ++launches_, kHertzCarry<<<gridFor(np), kBlock, 0, stream_>>>(d_, np, hzPrevCount_, hzPrevKeys_.p, hzPrevXi_.p, hzKeys_.p,
                                                       hzXi_.p);
@@ -2275,8 +2259,6 @@ void Sim<R>::hertzRebuildPairs(R skin) {
   }
   hzNumPairs_ = np;
   cudaCheck(cudaMemcpyAsync(hzRefPos_.p, pos_.p, numReal_ * sizeof(Q4<R>), cudaMemcpyDeviceToDevice, stream_), "D2D");
-  // pair incidence per body (pair order), reused until the next rebuild
-  buildIncidence(3, np, numReal_);
 }
 // src/solver_hertz.hpp:343-370
 template <class R>
@@ -2333,8 +2315,13 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
   const R skin = skinFrac * minRad;
   const R rebuildAt = R(0.25) * skin * skin;
   bool rebuild = hzNumPairs_ < 0;
-  if (!rebuild)  // the incidence buffers are shared with the XPBD step: rebuild them for this call
-    buildIncidence(3, hzNumPairs_, numReal_);
+  hzHead_.ensure(std::max(n, 1), false, stream_);
+  cudaCheck(cudaMemsetAsync(hzHead_.p, 0xff, std::max(n, 1) * sizeof(int), stream_), "memset");
+  if (!rebuild && hzNumPairs_ > 0)  // the shape may have changed since: every history may be set
+    cudaCheck(cudaMemsetAsync(hzOn_.p, 0xff, (hzNumPairs_ / 32 + 1) * sizeof(unsigned), stream_), "memset");
+  hzPosRad_.ensure(std::max(n, 1), false, stream_);
+  if (n > 0)
+    ++launches_, kHertzPosRad<<<gridFor(n), kBlock, 0, stream_>>>(d_, n, hzPosRad_.p);
   const bool hasShapes = shape_.numPoints > 0;
   const int nw = (int)wallsHost_.size();
   HertzP<R> P{dt, eN_, mu_, gs_, hzContactFrac_, nw};
@@ -2353,13 +2340,14 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
     qA_.ensure(std::max(np, 1), false, stream_);
     qB_.ensure(std::max(np, 1), false, stream_);
     qC_.ensure(std::max(np, 1), false, stream_);
-    iE_.ensure(std::max(np, 1), false, stream_);
+    const HertzChains chains{hzHead_.p, hzNext_.p};
     if (np > 0) {
       if (hasShapes)
         ++launches_, kHertzShapePairs<<<gridFor(np), kBlock, 0, stream_>>>(d_, np, P, hzXi_.p, hzSnPair_.p, qA_.p, qB_.p, qC_.p,
-                                                               iE_.p);
+                                                               chains);
       else
-        ++launches_, kHertzPairs<<<gridFor(np), kBlock, 0, stream_>>>(d_, np, P, hzXi_.p, qA_.p, qB_.p, qC_.p, iE_.p);
+        ++launches_, kHertzPairs<<<gridFor(np, kHertzTile), kBlock, 0, stream_>>>(d_, np, P, hzPosRad_.p, hzOn_.p, hzXi_.p, qA_.p,
+                                                                           qB_.p, qC_.p, chains);
       KCHECK("hertz pairs");
     }
     const int nc = (nw > 0) ? hzNumWallCand_ : 0;
@@ -2374,8 +2362,8 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
     mark(ST_HERTZ_INTEGRATE);
     if (n > 0) {
       ++launches_, kHertzGatherIntegrate<<<gridFor(n), kBlock, 0, stream_>>>(
-          d_, n, incOff_.p, incValsS_.p, qA_.p, qB_.p, qC_.p, iE_.p, nc > 0 ? hzCandOff_.p : nullptr, nc, hzFW_.p,
-          hzTW_.p, hzOnW_.p, g, dt, hasShapes ? 1 : 0);
+          d_, n, chains, qA_.p, qB_.p, qC_.p, nc > 0 ? hzCandOff_.p : nullptr, nc, hzFW_.p, hzTW_.p, hzOnW_.p, g, dt,
+          hasShapes ? 1 : 0, k == 0 ? 1 : 0, hzPosRad_.p);
       KCHECK("hertz integrate");
     }
     if ((k & 15) == 15 || k == nsteps - 1) {

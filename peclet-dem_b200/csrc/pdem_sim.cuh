@@ -340,6 +340,9 @@ class Sim {
   DBuf<Q4<R>> hzXi_, hzPrevXi_, hzXiWall_, hzRefPos_;
   DBuf<u64> hzKeys_, hzPrevKeys_;
   DBuf<R> hzSnPair_, hzSnWall_;
+  DBuf<unsigned> hzOn_;          // pairs whose history may be set, a bit each
+  DBuf<int> hzHead_, hzNext_;    // the bodies' chains of touching pairs
+  DBuf<Q4<R>> hzPosRad_;         // positions with radii
   DBuf<int> hzWallCand_, hzCandOff_, hzOnW_;
   DBuf<Q4<R>> hzFW_, hzTW_;
   struct Mark {

@@ -1161,10 +1161,9 @@ __global__ void kPosJacobiGather(Dev<R> d, int n, Incidence inc, const Q4<R>* co
 // incidence entries: entry 2i = (body of side A, i<<1), 2i+1 = (body of side B, i<<1|1) or none
 template <class R, int KIND>
 __global__ void kIncidenceKeys(Dev<R> d, int ne, int* keys, int* vals, int none) {
-  // KIND 0: manifolds by real body; 1: contacts by real body; 2: contacts by raw slot;
-  // 3: candidate pairs by raw slot
+  // KIND 0: manifolds by real body; 1: contacts by real body; 2: contacts by raw slot
   GRID_STRIDE(i, ne) {
-    int2 ab = (KIND == 0) ? d.mab[i] : (KIND == 3 ? d.pairs[i] : d.cab[i]);
+    int2 ab = (KIND == 0) ? d.mab[i] : d.cab[i];
     int a = ab.x, b = ab.y;
     if (KIND == 0 || KIND == 1) {
       a = d.realIdx[a];
