@@ -6,8 +6,8 @@
 // The saturated colour as levels: consecutive contacts of one body pair form a run, and a run's level
 // is one above the latest earlier run that shares a body. Runs of a level are body-disjoint and every
 // body meets its runs in contact order, so the levels in turn, each run in its own order, give the
-// serial result bit for bit. A warp takes a run: its lanes hold 32 contacts' records and update the two
-// bodies' positions in registers, one contact after the other.
+// serial result bit for bit. Half a warp takes a run (some 15 contacts of a pair): its lanes hold 16
+// contacts' records and update the two bodies' positions in registers, one contact after the other.
 //
 // One persistent launch runs all sweeps: the colours, the levels and the Jacobi phases, with a barrier
 // after each. ONE: one block with every body's position in shared memory (a barrier costs tens of
@@ -192,10 +192,11 @@ __device__ __forceinline__ bool denseUpdate(const DenseRec<R>& c, V3<R>& pA, V3<
   runMax(mx, -C);
   return true;
 }
+constexpr int kDenseLanes = 16;  // lanes of a run
 template <class R>
-__device__ __forceinline__ V3<R> denseShfl(V3<R> v, int lane) {
-  return V3<R>{__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
-               __shfl_sync(0xffffffffu, v.z, lane)};
+__device__ __forceinline__ V3<R> denseShfl(unsigned mask, V3<R> v, int lane) {
+  return V3<R>{__shfl_sync(mask, v.x, lane, kDenseLanes), __shfl_sync(mask, v.y, lane, kDenseLanes),
+               __shfl_sync(mask, v.z, lane, kDenseLanes)};
 }
 
 // left: uncoloured contacts, their incidence lists by body (entries l << 1 | side); corr, ok: [left]
@@ -257,12 +258,14 @@ __global__ void __launch_bounds__(kDenseBlock) kDenseSweeps(Dev<R> d, const int*
     }
     for (int lv = 0; lv < levels; ++lv) {  // the saturated colour
       const int r1 = D.lvOff[lv + 1];
-      for (long k = D.lvOff[lv] + (gtid >> 5); k < r1; k += gstride >> 5) {
+      const int sub = lane % kDenseLanes;
+      const unsigned group = ((1u << kDenseLanes) - 1u) << (lane - sub);
+      for (long k = D.lvOff[lv] + gtid / kDenseLanes; k < r1; k += gstride / kDenseLanes) {
         const int run = D.order[k], s = D.start[run], e = D.start[run + 1];
         V3<R> p0{0, 0, 0}, p1{0, 0, 0};  // the run's bodies, in its first contact's order
         int A = 0, B = -1;
-        for (int t0 = s; t0 < e; t0 += 32) {
-          const int t = t0 + lane, m = min(32, e - t0);
+        for (int t0 = s; t0 < e; t0 += kDenseLanes) {
+          const int t = t0 + sub, m = min(kDenseLanes, e - t0);
           DenseRec<R> q{};
           R lam = R(0);
           if (t < e) {
@@ -270,8 +273,8 @@ __global__ void __launch_bounds__(kDenseBlock) kDenseSweeps(Dev<R> d, const int*
             lam = d.posLamC[q.id.x];
           }
           if (t0 == s) {
-            A = __shfl_sync(0xffffffffu, q.id.y, 0);
-            B = __shfl_sync(0xffffffffu, q.id.z, 0);
+            A = __shfl_sync(group, q.id.y, 0, kDenseLanes);
+            B = __shfl_sync(group, q.id.z, 0, kDenseLanes);
             p0 = at(A);
             if (B >= 0)
               p1 = at(B);
@@ -279,16 +282,16 @@ __global__ void __launch_bounds__(kDenseBlock) kDenseSweeps(Dev<R> d, const int*
           const bool swap = t < e && q.id.y != A;
           for (int j = 0; j < m; ++j) {
             V3<R> a = swap ? p1 : p0, b = swap ? p0 : p1;
-            if (lane == j) {
+            if (sub == j) {
               R dl;
               if (denseUpdate(q, a, b, dl, mx))
                 d.posLamC[q.id.x] = lam + dl;
             }
-            p0 = denseShfl(swap ? b : a, j);
-            p1 = denseShfl(swap ? a : b, j);
+            p0 = denseShfl(group, swap ? b : a, j);
+            p1 = denseShfl(group, swap ? a : b, j);
           }
         }
-        if (lane == 0) {
+        if (sub == 0) {
           pos[A] = q4(p0);
           if (B >= 0)
             pos[B] = q4(p1);
