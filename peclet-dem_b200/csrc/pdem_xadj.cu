@@ -496,27 +496,44 @@ __device__ __forceinline__ void posIn(const XScene& sc, const XView& r, const XW
   put3(in, 28, w.cgB[k]);
 }
 
+__device__ __forceinline__ void posFwdEntry(const XScene& sc, const XView& r, const XWork& w, int k, int sweep, int tag,
+                                            u64& hs) {
+  const int2 ab = r.cab[k];
+  const D4 xA = w.xP[ab.x], xB = ab.y >= 0 ? w.xP[ab.y] : D4{0, 0, 0, 0};
+  D4* tape = w.tp + 2 * ((long)sweep * r.nc + k);
+  tape[0] = xA;
+  tape[1] = xB;
+  double in[kPosIn], out[kPosOut];
+  posIn(sc, r, w, k, ab, xA, xB, in);
+  unsigned bits = 0;
+  posMap<double>(in, out, posC(sc, ab), w.hash ? &bits : nullptr);
+  if (w.hash)
+    hs += mixWord(((u64)(unsigned)tag << 40) ^ ((u64)(unsigned)(sweep + 4096) << 28) ^ ((u64)(unsigned)k << 8) ^ bits);
+  w.xP[ab.x] = get3(out, 0);
+  if (ab.y >= 0)
+    w.xP[ab.y] = get3(out, 3);
+  w.posLam[k] += out[6];
+}
 __global__ void kxPos(XScene sc, XView r, XWork w, int col, int sweep, int tag) {
   const int b = r.cOff[col], cnt = r.cOff[col + 1] - b;
   u64 hs = 0;
-  GRID_STRIDE(t, cnt) {
-    const int k = r.cOrder[b + t];
-    const int2 ab = r.cab[k];
-    const D4 xA = w.xP[ab.x], xB = ab.y >= 0 ? w.xP[ab.y] : D4{0, 0, 0, 0};
-    D4* tape = w.tp + 2 * ((long)sweep * r.nc + k);
-    tape[0] = xA;
-    tape[1] = xB;
-    double in[kPosIn], out[kPosOut];
-    posIn(sc, r, w, k, ab, xA, xB, in);
-    unsigned bits = 0;
-    posMap<double>(in, out, posC(sc, ab), w.hash ? &bits : nullptr);
-    if (w.hash)
-      hs += mixWord(((u64)(unsigned)tag << 40) ^ ((u64)(unsigned)(sweep + 4096) << 28) ^ ((u64)(unsigned)k << 8) ^ bits);
-    w.xP[ab.x] = get3(out, 0);
-    if (ab.y >= 0)
-      w.xP[ab.y] = get3(out, 3);
-    w.posLam[k] += out[6];
-  }
+  GRID_STRIDE(t, cnt) { posFwdEntry(sc, r, w, r.cOrder[b + t], sweep, tag, hs); }
+  if (w.hash)
+    warpHashAdd(w.hash, hs);
+}
+// the replay's position sweeps in one persistent cluster launch, as kxPgsCluster: a launch a colour and
+// sweep cost 7 us each (90 a substep on a packed bed)
+__global__ void __launch_bounds__(kB) kxPosCluster(XScene sc, XView r, XWork w, int sweeps, int tag) {
+  const int nb = gridDim.x;
+  u64 hs = 0;
+  for (int it = 0; it < sweeps; ++it)
+    for (int c = 0; c < r.ncolP; ++c) {
+      const int b = r.cOff[c], cnt = r.cOff[c + 1] - b;
+      const int lo = (int)((long)cnt * blockIdx.x / nb), hi = (int)((long)cnt * (blockIdx.x + 1) / nb);
+      for (int t = lo + threadIdx.x; t < hi; t += blockDim.x)
+        posFwdEntry(sc, r, w, r.cOrder[b + t], it, tag, hs);
+      cg::this_cluster().sync();
+    }
   if (w.hash)
     warpHashAdd(w.hash, hs);
 }
@@ -606,35 +623,47 @@ __global__ void __launch_bounds__(kBR) kxPosRev(XScene sc, XView r, XWork w, int
 // the hand-written reverses of the position update, the warm start and the approach velocity:
 // one entry a thread (the grouped kernels above and below reverse the same maps through
 // forward-mode chunks: the cross-check)
+__device__ __forceinline__ void posRevEntry(const XScene& sc, const XView& r, const XWork& w, int k, int sweep) {
+  const int2 ab = r.cab[k];
+  const D4* tape = w.tp + 2 * ((long)sweep * r.nc + k);
+  double in[kPosIn], yb[kPosOut], xb[kPosIn];
+  posIn(sc, r, w, k, ab, tape[0], tape[1], in);
+  for (int j = 0; j < kPosOut; ++j)
+    yb[j] = 0.0;
+  put3(yb, 0, w.axP[ab.x]);
+  if (ab.y >= 0)
+    put3(yb, 3, w.axP[ab.y]);
+  yb[6] = w.aposLam[k];
+  for (int j = 0; j < kPosIn; ++j)
+    xb[j] = 0.0;
+  posRev(in, yb, xb, posC(sc, ab));
+  w.axP[ab.x] = get3(xb, 0);
+  add4(w.aqP[ab.x], xb + 6);
+  add4(w.aq[ab.x], xb + 14);
+  if (ab.y >= 0) {
+    w.axP[ab.y] = get3(xb, 3);
+    add4(w.aqP[ab.y], xb + 10);
+    add4(w.aq[ab.y], xb + 18);
+  }
+  add3(w.acgN[k], xb + 22);
+  add3(w.acgA[k], xb + 25);
+  add3(w.acgB[k], xb + 28);
+}
 __global__ void kxPosRevH(XScene sc, XView r, XWork w, int col, int sweep) {
   const int b = r.cOff[col], cnt = r.cOff[col + 1] - b;
-  GRID_STRIDE(t, cnt) {
-    const int k = r.cOrder[b + t];
-    const int2 ab = r.cab[k];
-    const D4* tape = w.tp + 2 * ((long)sweep * r.nc + k);
-    double in[kPosIn], yb[kPosOut], xb[kPosIn];
-    posIn(sc, r, w, k, ab, tape[0], tape[1], in);
-    for (int j = 0; j < kPosOut; ++j)
-      yb[j] = 0.0;
-    put3(yb, 0, w.axP[ab.x]);
-    if (ab.y >= 0)
-      put3(yb, 3, w.axP[ab.y]);
-    yb[6] = w.aposLam[k];
-    for (int j = 0; j < kPosIn; ++j)
-      xb[j] = 0.0;
-    posRev(in, yb, xb, posC(sc, ab));
-    w.axP[ab.x] = get3(xb, 0);
-    add4(w.aqP[ab.x], xb + 6);
-    add4(w.aq[ab.x], xb + 14);
-    if (ab.y >= 0) {
-      w.axP[ab.y] = get3(xb, 3);
-      add4(w.aqP[ab.y], xb + 10);
-      add4(w.aq[ab.y], xb + 18);
+  GRID_STRIDE(t, cnt) { posRevEntry(sc, r, w, r.cOrder[b + t], sweep); }
+}
+// all of them in one persistent cluster launch (10 us a launch before)
+__global__ void __launch_bounds__(kB) kxPosRevCluster(XScene sc, XView r, XWork w, int sweeps) {
+  const int nb = gridDim.x;
+  for (int it = sweeps - 1; it >= 0; --it)
+    for (int c = r.ncolP - 1; c >= 0; --c) {
+      const int b = r.cOff[c], cnt = r.cOff[c + 1] - b;
+      const int lo = (int)((long)cnt * blockIdx.x / nb), hi = (int)((long)cnt * (blockIdx.x + 1) / nb);
+      for (int t = lo + threadIdx.x; t < hi; t += blockDim.x)
+        posRevEntry(sc, r, w, r.cOrder[b + t], it);
+      cg::this_cluster().sync();
     }
-    add3(w.acgN[k], xb + 22);
-    add3(w.acgA[k], xb + 25);
-    add3(w.acgB[k], xb + 28);
-  }
 }
 // over every manifold in one launch: the body adjoints it reads are the sweeps' (not changed
 // here), and its orientation adjoints accumulate with atomics
@@ -1551,9 +1580,11 @@ struct XAdjAccess {
     kxIntegrate<<<gn, kB, 0, st>>>(sc, r, w);
     if (R.nc > 0) {
       cudaCheck(cudaMemsetAsync(w.posLam, 0, R.nc * sizeof(double), st), "memset");
-      for (int it = 0; it < R.posSweeps; ++it)
-        for (int c = 0; c < R.ncolP; ++c)
-          kxPos<<<gc, kB, 0, st>>>(sc, r, w, c, it, tag);
+      if (!(R.nc <= kClusterEntries && R.ncolP > 0 &&
+            launchOneCluster(kxPosCluster, kClusterBlocks, kB, st, sc, r, w, R.posSweeps, tag)))
+        for (int it = 0; it < R.posSweeps; ++it)
+          for (int c = 0; c < R.ncolP; ++c)
+            kxPos<<<gc, kB, 0, st>>>(sc, r, w, c, it, tag);
     }
     if (next)
       kxCheck<<<gn, kB, 0, st>>>(sc, view(*next), w);
@@ -1577,7 +1608,8 @@ struct XAdjAccess {
     const int gnG = gridFor((long)kGroup * n, kBR), gcG = gridFor((long)kGroup * std::max(R.nc, 1), kBR),
               gmG = gridFor((long)kGroup * std::max(R.nm, 1), kBR);
     kxRevInit<<<gridFor(std::max(n, std::max(R.nc, R.nm))), kB, 0, st>>>(sc, r, w);
-    if (R.nc > 0)
+    if (R.nc > 0 && !(!A.dualCheck && R.nc <= kClusterEntries && R.ncolP > 0 &&
+                      launchOneCluster(kxPosRevCluster, kClusterBlocks, kB, st, sc, r, w, R.posSweeps)))
       for (int it = R.posSweeps - 1; it >= 0; --it)
         for (int c = R.ncolP - 1; c >= 0; --c)
           if (A.dualCheck)
