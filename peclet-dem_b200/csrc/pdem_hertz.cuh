@@ -72,16 +72,21 @@ struct HertzP {
   int numWalls;
 };
 
-// The touching pairs of each body as a chain in any order: head[body] (-1: none), next[2 pair + side].
+// The touching pairs of each of the n bodies as a chain in any order: head[body] (-1: none),
+// next[2 pair + side]. A list that the XPBD step wrote in between may name its ghost slots (n and up): they
+// exert forces, as in the reference, and take none.
 struct HertzChains {
   int *head, *next;
+  int n;
 };
 __device__ __forceinline__ void hertzLink(const HertzChains& H, int pair, int i, int j) {
-  H.next[2 * pair] = atomicExch(&H.head[i], 2 * pair);
-  H.next[2 * pair + 1] = atomicExch(&H.head[j], 2 * pair + 1);
+  if (i < H.n)
+    H.next[2 * pair] = atomicExch(&H.head[i], 2 * pair);
+  if (j < H.n)
+    H.next[2 * pair + 1] = atomicExch(&H.head[j], 2 * pair + 1);
 }
 
-// positions with radii, one load a body in the pair test
+// positions with radii of all body slots, one load a body in the pair test
 template <class R>
 __global__ void kHertzPosRad(Dev<R> d, int n, Q4<R>* pr) {
   GRID_STRIDE(i, n) {

@@ -2321,9 +2321,9 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
   cudaCheck(cudaMemsetAsync(hzHead_.p, 0xff, std::max(n, 1) * sizeof(int), stream_), "memset");
   if (!rebuild && hzNumPairs_ > 0)  // the shape may have changed since: every history may be set
     cudaCheck(cudaMemsetAsync(hzOn_.p, 0xff, (hzNumPairs_ / 32 + 1) * sizeof(unsigned), stream_), "memset");
-  hzPosRad_.ensure(std::max(n, 1), false, stream_);
+  hzPosRad_.ensure(std::max(capacity_, 1), false, stream_);
   if (n > 0)
-    ++launches_, kHertzPosRad<<<gridFor(n), kBlock, 0, stream_>>>(d_, n, hzPosRad_.p);
+    ++launches_, kHertzPosRad<<<gridFor(capacity_), kBlock, 0, stream_>>>(d_, capacity_, hzPosRad_.p);
   const bool hasShapes = shape_.numPoints > 0;
   const int nw = (int)wallsHost_.size();
   HertzP<R> P{dt, eN_, mu_, gs_, hzContactFrac_, nw};
@@ -2342,7 +2342,7 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
     qA_.ensure(std::max(np, 1), false, stream_);
     qB_.ensure(std::max(np, 1), false, stream_);
     qC_.ensure(std::max(np, 1), false, stream_);
-    const HertzChains chains{hzHead_.p, hzNext_.p};
+    const HertzChains chains{hzHead_.p, hzNext_.p, n};
     if (np > 0) {
       if (hasShapes)
         ++launches_, kHertzShapePairs<<<gridFor(np), kBlock, 0, stream_>>>(d_, np, P, hzXi_.p, hzSnPair_.p, qA_.p, qB_.p, qC_.p,

@@ -64,6 +64,30 @@ def test_hertz_vs_oracle(gpu_api, orc_api, name, mk, calls, substeps, skin, prec
         assert not bad, f"{name} {precision}: hertz call {k}: {bad[:4]}"
 
 
+@pytest.mark.parametrize("precision,rtol", [("fp32", 0.0), ("fp64", 1e-12)])
+def test_hertz_after_a_periodic_step(gpu_api, orc_api, precision, rtol):
+    """Both engines keep their candidate pairs in one list. A periodic XPBD step between two Hertz calls
+    leaves pairs with its ghost slots (numbers above the bodies') there, which the second call takes as it
+    finds them: forces on the bodies, none on the ghosts."""
+    sc = S.polydisperse_periodic()
+
+    def extra(s):
+        s.set_hertz_material(0, 1e7, 0.3)
+        s.enable_periodicity(False, False, False)
+    sc.planes = []
+    a, b = P.build(gpu_api, sc, extra, precision), P.build(orc_api, sc, extra, precision)
+    for s in (a, b):
+        s.step_hertz(2e-6, 4, 0.3)
+        s.enable_periodicity(True, True, False)
+        s.step(1e-6)
+        s.enable_periodicity(False, False, False)
+        pairs = s.debug_pairs()
+        assert pairs.max() >= sc.n
+        s.step_hertz(2e-6, 3, 0.3)
+    bad = P.diff(P.snapshot(a, products=False), P.snapshot(b, products=False), rtol=rtol)
+    assert not bad, bad[:4]
+
+
 def test_hertz_rejects_periodic(gpu_api):
     """The reference refuses the Hertz engine on periodic domains (src/sim.hpp:629-634); the B200
     step raises the same error type."""
