@@ -487,57 +487,29 @@ __device__ bool contactLaw(const Model<R>& M, int i, int j, int k, const T* in, 
 // forward: contact forces into F, T (atomics), new histories; then the kick-drift, which also
 // clears F, T for the next substep (they are cleared once at the window start)
 //
-// A few percent of the candidates touch, and the law needs some 100 registers: a block tests a tile of
-// candidates, kTileWays of them a thread so that their dependent loads (contact, radius, positions) are in
-// flight together, lists the touching ones in shared memory and then computes those with full warps.
-// 430,000 candidates of 131,072 spheres, FP64: 25.5 us as one thread a candidate.
-constexpr int kTileWays = 4, kTileF = 128, kTileB = 256;
-// touching candidates of tile [first, first + kTileWays * THREADS) into sList; apart(c) for the others
-template <int THREADS, class R, class APART>
-__device__ __forceinline__ int touching(const Model<R>& M, const StateView<R>& s, long first, int* sList, int* sCount,
-                                        APART&& apart) {
-  if (threadIdx.x == 0)
-    *sCount = 0;
-  __syncthreads();
-  bool on[kTileWays];
-#pragma unroll
-  for (int q = 0; q < kTileWays; ++q) {
-    const long c = first + q * THREADS + threadIdx.x;
-    on[q] = c < M.nc && contactActive(M, c, s);
-  }
-#pragma unroll
-  for (int q = 0; q < kTileWays; ++q) {
-    const long c = first + q * THREADS + threadIdx.x;
-    if (on[q])
-      sList[atomicAdd(sCount, 1)] = (int)c;
-    else if (c < M.nc)
-      apart(c);
-  }
-  __syncthreads();
-  return *sCount;
-}
+// One thread a candidate in blocks of 128: the touching ones (a few percent) need some 100 registers, and
+// small blocks keep more of them resident. Rollout and adjoint over boxes of 2,048 spheres, against blocks of
+// 256: FP64 1.01-1.06 times the speed from 2,048 to 131,072 spheres, FP32 1.01-1.03. (Tiles of 512
+// candidates whose touching ones are listed in shared memory and computed by full warps are equal at 131,072
+// spheres in FP64 and 0.86-0.95 of this speed below 65,536 spheres, both precisions: two block barriers on
+// each block's chain and a quarter of the threads.)
+constexpr int kForwardBlock = 128;
 template <class R>
-__global__ void __launch_bounds__(kTileF) kContacts(Model<R> M, StateView<R> s, StateView<R> t, R* F, R* T) {
-  __shared__ int sList[kTileWays * kTileF], sCount;
-  for (long first = (long)blockIdx.x * (kTileWays * kTileF); first < M.nc; first += (long)gridDim.x * (kTileWays * kTileF)) {
-    const int n = touching<kTileF>(M, s, first, sList, &sCount, [&](long c) { st3(t.xi, c, V3<R>{R(0), R(0), R(0)}); });
-    for (int q = threadIdx.x; q < n; q += kTileF) {
-      const long c = sList[q];
-      Contact<R> C;
-      contactPrimal(M, c, s, C);
-      if (!C.active) {  // cannot happen (the same test); kept for safety
-        st3(t.xi, c, V3<R>{R(0), R(0), R(0)});
-        continue;
-      }
-      st3(t.xi, c, C.xi3);
-      atomicAdd3(F, C.i, C.f);
-      atomicAdd3(T, C.i, cross(C.rA, C.f));
-      if (C.j >= 0) {
-        atomicAdd3(F, C.j, mul(C.f, R(-1)));
-        atomicAdd3(T, C.j, cross(C.rB, mul(C.f, R(-1))));
-      }
+__global__ void __launch_bounds__(kForwardBlock) kContacts(Model<R> M, StateView<R> s, StateView<R> t, R* F, R* T) {
+  GRID_STRIDE(c, M.nc) {
+    Contact<R> C;
+    contactPrimal(M, c, s, C);
+    if (!C.active) {
+      st3(t.xi, c, V3<R>{R(0), R(0), R(0)});
+      continue;
     }
-    __syncthreads();  // the list is read before the next tile's
+    st3(t.xi, c, C.xi3);
+    atomicAdd3(F, C.i, C.f);
+    atomicAdd3(T, C.i, cross(C.rA, C.f));
+    if (C.j >= 0) {
+      atomicAdd3(F, C.j, mul(C.f, R(-1)));
+      atomicAdd3(T, C.j, cross(C.rB, mul(C.f, R(-1))));
+    }
   }
 }
 // one thread per component (coalesced, three times the threads of one per sphere); the
@@ -589,23 +561,17 @@ __device__ inline void flushParams(double* thetaB, double gE, double ge, double 
 }
 // contact adjoints (hand reversal), in two passes so that the few touching contacts do not set
 // the occupancy of the many apart: the scan clears the history adjoint of every apart contact
-// and lists the touching ones, tile by tile (one counter update a tile); the second pass reverses the
-// listed contacts, its warps in lockstep so the parameter sums reduce with shuffles, in blocks of two warps
-// so that some thousand contacts spread over all SMs' FP64 pipes. It clears the other counter slot for the
-// next substep's scan. (Both in one kernel, at the reversal's 182 registers: 38 us against 30 for the two.)
+// and lists the touching ones (count[slot]); the second pass reverses the listed contacts, its
+// warps in lockstep so the parameter sums reduce with shuffles, in blocks of two warps so that some
+// thousand contacts spread over all SMs' FP64 pipes. It clears the other counter slot for the next
+// substep's scan. (Both in one kernel, at the reversal's 182 registers: 38 us against 30 for the two.)
 template <class R>
-__global__ void __launch_bounds__(kTileB) kContactsAdjScan(Model<R> M, StateView<R> s, StateView<R> b0, int* list,
-                                                           int* count) {
-  __shared__ int sList[kTileWays * kTileB], sCount, sBase;
-  for (long first = (long)blockIdx.x * (kTileWays * kTileB); first < M.nc; first += (long)gridDim.x * (kTileWays * kTileB)) {
-    // a cleared history does not depend on the old one
-    const int n = touching<kTileB>(M, s, first, sList, &sCount, [&](long c) { st3(b0.xi, c, V3<R>{R(0), R(0), R(0)}); });
-    if (threadIdx.x == 0 && n > 0)
-      sBase = atomicAdd(count, n);
-    __syncthreads();
-    for (int q = threadIdx.x; q < n; q += kTileB)
-      list[sBase + q] = sList[q];
-    __syncthreads();  // the list is read before the next tile's
+__global__ void kContactsAdjScan(Model<R> M, StateView<R> s, StateView<R> b0, int* list, int* count) {
+  GRID_STRIDE(c, M.nc) {
+    if (contactActive(M, c, s))
+      list[atomicAdd(count, 1)] = (int)c;
+    else
+      st3(b0.xi, c, V3<R>{R(0), R(0), R(0)});  // cleared history: no dependence on the old one
   }
 }
 constexpr int kReverseBlock = 64;
@@ -1143,7 +1109,7 @@ void forward(const pdem_hz_model* h, int steps, int store, R* traj, R* work, cud
     const size_t a = store ? k : (k & 1), b = store ? k + 1 : ((k + 1) & 1);
     const StateView<R> s = view(traj + S * a, M.n), t = view(traj + S * b, M.n);
     if (M.nc > 0)
-      kContacts<R><<<pdem::gridFor(M.nc, kTileWays * kTileF), kTileF, 0, st>>>(M, s, t, F, T);
+      kContacts<R><<<pdem::gridFor(M.nc, kForwardBlock), kForwardBlock, 0, st>>>(M, s, t, F, T);
     kIntegrate<R><<<pdem::gridFor(3L * M.n), pdem::kBlock, 0, st>>>(M, s, t, F, T);
   }
   if (!store && (steps & 1) == 0)  // the final state of a ping-pong run always ends in block 1
@@ -1175,7 +1141,7 @@ void backward(const pdem_hz_model* h, int steps, const R* traj, R* adj, double* 
     kIntegrateAdj<R><<<pdem::gridFor(3L * M.n), pdem::kBlock, 0, st>>>(M, b1, b0, Fb, Tb);
     if (M.nc > 0) {
       if (mode == 0) {
-        kContactsAdjScan<R><<<pdem::gridFor(M.nc, kTileWays * kTileB), kTileB, 0, st>>>(M, s, b0, list, cnt + (k & 1));
+        kContactsAdjScan<R><<<pdem::gridFor(M.nc), pdem::kBlock, 0, st>>>(M, s, b0, list, cnt + (k & 1));
         // the active list is a small part of the contacts: a grid of a few blocks per SM strides it
         const int g = std::min(pdem::gridFor(M.nc, kReverseBlock), 8 * pdem::kNumSMs);
         kContactsAdj<R><<<g, kReverseBlock, 0, st>>>(M, s, b1, b0, Fb, Tb, thetaB, list, cnt + (k & 1),
