@@ -225,6 +225,8 @@ int pdem_debug_reuse(pdem_handle h, long* out3);
 int pdem_debug_ranked(pdem_handle h, long* out2);
 /* device allocations made by this library's growable buffers since it was loaded */
 long pdem_debug_allocs(void);
+/* test hook: the k-th growable-buffer allocation from now throws as a failed one does (0: none) */
+int pdem_debug_refuse_alloc(long k);
 /* sweeps executed since profile_enable: velocity, stabilization, position; and substeps */
 int pdem_debug_sweeps(pdem_handle h, long* out4);
 

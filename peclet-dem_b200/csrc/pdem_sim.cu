@@ -25,6 +25,7 @@
 namespace pdem {
 
 long gDeviceAllocs = 0;
+long gRefuseAlloc = 0;
 static const int kOne = 1;  // H2D source of a device flag set from the host
 
 void cudaCheck(cudaError_t e, const char* what) {
@@ -2230,10 +2231,12 @@ void Sim<R>::setMaxContacts(int n) {
 template <class R>
 void Sim<R>::hertzCommitHistory() {
   const int n = hzNumPairs_;
-  if (n <= 0) {
-    hzPrevCount_ = 0;
+  if (n < 0)
+    return;  // committed before a rebuild that failed (or there was no list)
+  hzNumPairs_ = -1;  // the buffers hold no list until the rebuild has filled them
+  hzPrevCount_ = 0;
+  if (n == 0)
     return;
-  }
   // the list becomes the previous one as it stands (in pair order)
   std::swap(hzKeys_.p, hzPrevKeys_.p);
   std::swap(hzKeys_.n, hzPrevKeys_.n);

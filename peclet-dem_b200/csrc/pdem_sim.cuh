@@ -30,6 +30,8 @@ void cudaCheck(cudaError_t e, const char* what);
 
 // device allocations made by growable buffers since load (instrumentation)
 extern long gDeviceAllocs;
+// test hook: the allocation from now that is refused (0: none)
+extern long gRefuseAlloc;
 
 // growable device buffer (contents not preserved unless asked), allocated in stream order from the
 // device's default pool: growth neither waits for the device nor returns memory to the driver (the
@@ -53,6 +55,8 @@ struct DBuf {
     if (p && cap < n + n / 2)
       cap = n + n / 2;  // grow geometrically: counts that creep up each substep reallocate rarely
     T* q = nullptr;
+    if (gRefuseAlloc > 0 && --gRefuseAlloc == 0)
+      throw CudaError("device allocation refused (test hook)");
     ++gDeviceAllocs;
     cudaCheck(cudaMallocAsync(reinterpret_cast<void**>(&q), cap * sizeof(T), s), "cudaMallocAsync");
     cudaCheck(cudaMemsetAsync(q, 0, cap * sizeof(T), s), "cudaMemset");

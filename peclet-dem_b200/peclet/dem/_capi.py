@@ -113,6 +113,7 @@ _SIGS = {
     "profile_read_host": (C.c_int, [_vp, _dbl_p, C.c_int]),
     "debug_sweeps": (C.c_int, [_vp, _long_p]),
     "debug_allocs": (C.c_long, []),
+    "debug_refuse_alloc": (C.c_int, [C.c_long]),
     "timer_start": (C.c_int, [_vp]),
     "debug_reuse": (C.c_int, [_vp, _long_p]),
     "timer_stop": (C.c_int, [_vp, _dbl_p]),

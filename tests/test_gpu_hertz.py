@@ -88,6 +88,30 @@ def test_hertz_after_a_periodic_step(gpu_api, orc_api, precision, rtol):
     assert not bad, bad[:4]
 
 
+@pytest.mark.parametrize("precision,rtol", [("fp32", 0.0), ("fp64", 1e-12)])
+def test_failed_rebuild_keeps_the_engine_usable(gpu_api, orc_api, precision, rtol):
+    """A pair-list rebuild whose allocation fails (refused by a test hook) leaves no list behind: the next
+    call rebuilds it first and carries the histories over. The oracle's single call of 16 + 16 substeps, whose
+    rebuild falls between them, is the reference."""
+    sc, extra = _drum_spheres()
+    a, b = P.build(gpu_api, sc, extra, precision), P.build(orc_api, sc, extra, precision)
+    for s in (a, b):
+        s.step_hertz(2e-6, 8, 0.005)
+    b.step_hertz(2e-6, 32, 0.005)
+    gpu_api.fn["debug_refuse_alloc"](1)
+    try:
+        with pytest.raises(Exception, match="refused"):
+            a.step_hertz(2e-6, 32, 0.005)
+    finally:
+        gpu_api.fn["debug_refuse_alloc"](0)
+    assert len(a.debug_hertz()[0]) == 0
+    a.step_hertz(2e-6, 16, 0.005)
+    sa, sb = P.snapshot(a, products=False), P.snapshot(b, products=False)
+    (sa["hk"], sa["hx"]), (sb["hk"], sb["hx"]) = a.debug_hertz(), b.debug_hertz()
+    bad = P.diff(sa, sb, rtol=rtol)
+    assert not bad, bad[:4]
+
+
 def test_hertz_rejects_periodic(gpu_api):
     """The reference refuses the Hertz engine on periodic domains (src/sim.hpp:629-634); the B200
     step raises the same error type."""
