@@ -535,19 +535,24 @@ __global__ void __launch_bounds__(kFlowBlock, 1) kFlowSweeps(Dev<R> d, const int
         plam = rec.lam[item.x + gt];
     }
   };
-  // wait for this warp's copy
-  auto landed = [&] {
+  // wait for this warp's copy, if one is outstanding; a copy that is late stays so: the warp takes no more
+  // records, and waits for it once more at the end
+  auto landed = [&](long limit) {
+    if (!pending)
+      return;
     long spins = 0;
     bool late = false;
     while (!late && !flowBulkDone(bar, parity))
-      late = ++spins > kBarrierSpins;
+      late = ++spins > limit;
     if (late) {
       atomicOr(gb.err, kErrBarrier);
       dead = true;
     }
-    lost = __any_sync(0xffffffffu, late || lost);
-    parity ^= 1u;
-    pending = false;
+    lost = __any_sync(0xffffffffu, late);
+    if (!lost) {
+      parity ^= 1u;
+      pending = false;
+    }
   };
   auto slot = [&](int k) {  // slot k of this thread's staged record
     Q4<R> v;
@@ -709,7 +714,8 @@ __global__ void __launch_bounds__(kFlowBlock, 1) kFlowSweeps(Dev<R> d, const int
         continue;
       }
       const long t = item.x + gt;
-      landed();
+      if (!lost)
+        landed(gb.spins);
       const bool act = gt < item.y && !lost;  // without its record an entry is left out
       // the previous sweep's stop, before anything of this one is stored: for entries of the first colour,
       // whose states come from that sweep, after their update (below); for others before they wait for
@@ -872,8 +878,8 @@ __global__ void __launch_bounds__(kFlowBlock, 1) kFlowSweeps(Dev<R> d, const int
     last = decide(iters - 1);
     stop = KIND == 2 ? (last < thr) : (last <= thr);
   }
-  if (pending)  // the copy of the item after the stop: it must land before this block's memory goes
-    landed();
+  // the copy of the item after the stop, or a late one: it must land before this block's memory goes
+  landed(kBarrierSpins);
   if (CLUSTER)
     cg::this_cluster().sync();  // no block leaves while another may write to its shared memory
   if (blk == 0 && tid == 0) {

@@ -65,6 +65,37 @@ def test_flow_own_image(gpu_api, monkeypatch, precision):
     assert a.counters()["manifolds"] > 5
 
 
+@pytest.mark.parametrize("entries", [None, 0], ids=["cluster", "grid"])
+def test_flow_time_out(gpu_api, orc_api, monkeypatch, entries):
+    """Every wait of the flow gives up after one poll (a record's copy, a state, the sweep's maximum): no
+    wait is repeated after that, so a loop of 600 sweeps ends at once, the step reports the error, and with
+    the default limit the next substeps match the oracle."""
+    import time
+    if entries is not None:
+        monkeypatch.setenv("PDEM_SWEEP_CLUSTER_ENTRIES", str(entries))
+    sc = _bed(700, (10, 600))
+    sim = P.build(gpu_api, sc, None, "fp64")
+    sim.debug_set_barrier_spins(1)
+    t = time.monotonic()
+    with pytest.raises(RuntimeError, match="barrier"):
+        for _ in range(3):
+            sim.step(sc.dt)
+    assert time.monotonic() - t < 5.0  # 600 sweeps of some 10 items at a microsecond or two, and the launches
+    sim.debug_set_barrier_spins(0)
+    sc.iterations = (10, 10)
+    sim.set_solver_iterations(*sc.iterations)
+    sim.set_positions(sc.pos)
+    sim.set_velocities(sc.vel)
+    sim.set_inv_mass(sc.inv_mass)
+    sim.set_inv_inertia(sc.inv_inertia)
+    ref = P.build(orc_api, sc, None, "fp64")
+    for k in range(3):
+        sim.step(sc.dt)
+        ref.step(sc.dt)
+        bad = P.diff(P.snapshot(sim), P.snapshot(ref), rtol=1e-12)
+        assert not bad, f"after the time-out, substep {k}: {bad[:4]}"
+
+
 def _stacked(n, points, seed=7):
     """Hollow cylinders side by side with a small tilt: tens of shell-point contacts a pair."""
     rng = np.random.default_rng(seed)
