@@ -1,8 +1,8 @@
 // Hertz-Mindlin soft-sphere engine (src/solver_hertz.hpp:41-606, src/sim.hpp:545-750).
 //
 // Explicit force model on a cached Verlet pair list: a touching pair's force, torques and Mindlin history
-// are computed by one thread, which links the pair into its two bodies' chains; each body then takes its
-// chain's contributions in pair order and its wall contributions in wall order (the reference's atomic
+// are computed by one thread, which notes the pair with its two bodies; each body then takes its
+// pairs' contributions in pair order and its wall contributions in wall order (the reference's atomic
 // order in the serial build), then a symplectic kick-drift. The pair list is rebuilt when any body moved half the skin; the shear
 // history is carried across rebuilds by pair key (sorted keys + binary search).
 #pragma once
@@ -72,18 +72,72 @@ struct HertzP {
   int numWalls;
 };
 
-// The touching pairs of each of the n bodies as a chain in any order: head[body] (-1: none),
-// next[2 pair + side]. A list that the XPBD step wrote in between may name its ghost slots (n and up): they
-// exert forces, as in the reference, and take none.
-struct HertzChains {
-  int *head, *next;
+// The touching pairs of each of the n bodies (2 pair + side), in any order: cnt[body] of them at slot +
+// off[body], where the body has room for all its pairs of the list; sorted: the same room, for the ones of a
+// body of many pairs in order; many: the blocks of kBlock bodies with one that has room for more than
+// kHertzScan. A list that the XPBD step wrote in between may name its ghost slots (n and up): they exert
+// forces, as in the reference, and take none.
+constexpr int kHertzSort = 8, kHertzScan = 32;
+struct HertzTouch {
+  int* cnt;
+  const int* off;
+  int *slot, *sorted;
+  const uint8_t* many;
   int n;
 };
-__device__ __forceinline__ void hertzLink(const HertzChains& H, int pair, int i, int j) {
+__device__ __forceinline__ void hertzNote(const HertzTouch& H, int pair, int i, int j) {
   if (i < H.n)
-    H.next[2 * pair] = atomicExch(&H.head[i], 2 * pair);
+    H.slot[H.off[i] + atomicAdd(&H.cnt[i], 1)] = 2 * pair;
   if (j < H.n)
-    H.next[2 * pair + 1] = atomicExch(&H.head[j], 2 * pair + 1);
+    H.slot[H.off[j] + atomicAdd(&H.cnt[j], 1)] = 2 * pair + 1;
+}
+// pairs of each body in a list that the XPBD step wrote (a rebuild's kHertzCarry counts its own)
+template <class R>
+__global__ void kHertzCount(Dev<R> d, int np, int n, int* cnt) {
+  GRID_STRIDE(idx, np) {
+    const int2 ij = d.pairs[idx];
+    if (ij.x < n)
+      atomicAdd(&cnt[ij.x], 1);
+    if (ij.y < n)
+      atomicAdd(&cnt[ij.y], 1);
+  }
+}
+// room for each body's pairs, in any order of the bodies (taken: used so far); the counts start again
+static __global__ void __launch_bounds__(kBlock) kHertzRoom(int n, int* cnt, int* off, int* taken, uint8_t* many) {
+  __shared__ int sWarp[kBlock / 32];
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (long b0 = (long)blockIdx.x * kBlock; b0 < n; b0 += (long)gridDim.x * kBlock) {
+    const long b = b0 + tid;
+    const int want = b < n ? cnt[b] : 0;
+    int x = want;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o)
+        x += y;
+    }
+    if (lane == 31)
+      sWarp[tid >> 5] = x;
+    const int any = __syncthreads_or(want > kHertzScan);
+    if (tid == 0) {
+      int sum = 0;
+      for (int w = 0; w < kBlock / 32; ++w)
+        sum += sWarp[w];
+      int at = atomicAdd(taken, sum);
+      for (int w = 0; w < kBlock / 32; ++w) {
+        const int c = sWarp[w];
+        sWarp[w] = at;
+        at += c;
+      }
+      many[b0 / kBlock] = any != 0;
+    }
+    __syncthreads();
+    if (b < n) {
+      off[b] = sWarp[tid >> 5] + x - want;
+      cnt[b] = 0;
+    }
+    __syncthreads();  // the warps' places are read before the next ones
+  }
 }
 
 // positions with radii of all body slots, one load a body in the pair test
@@ -104,7 +158,7 @@ __global__ void kHertzPosRad(Dev<R> d, int n, Q4<R>* pr) {
 constexpr int kHertzWays = 4, kHertzTile = kHertzWays * kBlock;
 template <class R>
 __global__ void __launch_bounds__(kBlock) kHertzPairs(Dev<R> d, int np, HertzP<R> P, const Q4<R>* pr, unsigned* on,
-                                                      Q4<R>* xi, Q4<R>* F, Q4<R>* TA, Q4<R>* TB, HertzChains H) {
+                                                      Q4<R>* xi, Q4<R>* F, Q4<R>* TA, Q4<R>* TB, HertzTouch H) {
   __shared__ int sList[kHertzTile], sCount;
   for (long first = (long)blockIdx.x * kHertzTile; first < np; first += (long)gridDim.x * kHertzTile) {
     if (threadIdx.x == 0)
@@ -168,7 +222,7 @@ __global__ void __launch_bounds__(kBlock) kHertzPairs(Dev<R> d, int np, HertzP<R
       F[idx] = q4(f);
       TA[idx] = q4(cross(rA, f));
       TB[idx] = q4(cross(rB, mul(f, R(-1))));
-      hertzLink(H, idx, i, j);
+      hertzNote(H, idx, i, j);
     }
     __syncthreads();  // the list is read before the next tile's
   }
@@ -177,7 +231,7 @@ __global__ void __launch_bounds__(kBlock) kHertzPairs(Dev<R> d, int np, HertzP<R
 // point-shell pairs (src/solver_hertz.hpp:454-606), one thread per pair (ordered sums over points)
 template <class R>
 __global__ void kHertzShapePairs(Dev<R> d, int np, HertzP<R> P, Q4<R>* xi, R* snPrev, Q4<R>* F, Q4<R>* TA, Q4<R>* TB,
-                                 HertzChains H) {
+                                 HertzTouch H) {
   const ShapeDesc<R> dA = d.shapes[0], dB = d.shapes[0];
   GRID_STRIDE(idx, np) {
     const int2 pr = d.pairs[idx];
@@ -275,7 +329,7 @@ __global__ void kHertzShapePairs(Dev<R> d, int np, HertzP<R> P, Q4<R>* xi, R* sn
     F[idx] = q4(fAcc);
     TA[idx] = q4(tA);
     TB[idx] = q4(tB);
-    hertzLink(H, (int)idx, A, B);
+    hertzNote(H, (int)idx, A, B);
   }
 }
 
@@ -434,17 +488,26 @@ __global__ void kHertzWalls(Dev<R> d, int ncand, HertzP<R> P, const int* cand, Q
 
 // per body: pair contributions in pair order, then wall contributions in wall order; then the
 // symplectic kick-drift (src/solver_hertz.hpp:374-425) with the forces consumed. first: the call's first
-// substep, which takes over what the delta arrays hold (normally zero) and clears them. A chain of up to
-// kHertzSort pairs is sorted in registers; a longer one is taken by repeated minimum. The chains replace a
-// walk over the body's whole incidence list (some 12 pairs, a flag each): 43 us of 262,144 spheres, FP32.
-constexpr int kHertzSort = 8;
+// substep, which takes over what the delta arrays hold (normally zero) and clears them. Up to kHertzSort
+// pairs of a body are sorted in registers, up to kHertzScan taken by repeated minimum; the pairs of a larger
+// grain are ranked by its whole block and summed in that order, one component a thread.
+// Before, a thread walked its body's whole incidence list (some 12 pairs, a flag each): 43 us of 262,144
+// spheres, FP32. A call of 40 substeps with one grain of 5 R (147 touching) among 3,000, FP64: 6.3-6.7 ms by
+// that walk, 4.2 so (19.7 by repeated minimum over a chain of all its pairs); eight such among 20,000: 8.3
+// and 5.8.
 template <class R>
-__global__ void kHertzGatherIntegrate(Dev<R> d, int n, HertzChains H, const Q4<R>* F, const Q4<R>* TA, const Q4<R>* TB,
-                                      const int* candOff, int ncand, const Q4<R>* FW, const Q4<R>* TW, const int* onW,
-                                      V3<R> g, R dt, int orient, int first, Q4<R>* pr) {
-  GRID_STRIDE(i, n) {
+__global__ void __launch_bounds__(kBlock) kHertzGatherIntegrate(Dev<R> d, int n, HertzTouch H, const Q4<R>* F,
+                                                                const Q4<R>* TA, const Q4<R>* TB, const int* candOff,
+                                                                int ncand, const Q4<R>* FW, const Q4<R>* TW,
+                                                                const int* onW, V3<R> g, R dt, int orient, int first,
+                                                                Q4<R>* pr) {
+  __shared__ R sVal[6][kBlock + 1], sSum[2][6];
+  __shared__ int sMany[kBlock], sManys;
+  const int tid = threadIdx.x;
+  for (long base = (long)blockIdx.x * kBlock; base < n; base += (long)gridDim.x * kBlock) {
+    const long i = base + tid;
     V3<R> f{0, 0, 0}, t{0, 0, 0};
-    if (first) {
+    if (first && i < n) {
       // the reference accumulates into the (normally zero) delta arrays it uses as force/torque
       f = v3(d.dVel[i]);
       t = v3(d.dAngVel[i]);
@@ -461,42 +524,90 @@ __global__ void kHertzGatherIntegrate(Dev<R> d, int n, HertzChains H, const Q4<R
         t = add(t, v3(TB[idx]));
       }
     };
-    const int head = H.head[i];
-    if (head >= 0) {
-      int node[kHertzSort];
-#pragma unroll
-      for (int k = 0; k < kHertzSort; ++k)
-        node[k] = INT_MAX;
-      int count = 0;
-      for (int q = head; q >= 0 && count <= kHertzSort; q = H.next[q], ++count) {
-        int v = q;
+    const bool many = H.many[base / kBlock] != 0;  // uniform over the block
+    const int count = i < n ? H.cnt[i] : 0;
+    if (count > 0 && count <= kHertzScan) {
+      const int* mine = H.slot + H.off[i];
+      if (count <= kHertzSort) {
+        int node[kHertzSort];
 #pragma unroll
         for (int k = 0; k < kHertzSort; ++k)
-          if (v < node[k]) {
-            const int w = node[k];
-            node[k] = v;
-            v = w;
+          node[k] = k < count ? mine[k] : INT_MAX;
+#pragma unroll
+        for (int p = 1; p < kHertzSort; ++p)
+#pragma unroll
+          for (int k = p; k > 0; --k) {
+            const int lo = min(node[k - 1], node[k]), hi = max(node[k - 1], node[k]);
+            node[k - 1] = lo;
+            node[k] = hi;
           }
-      }
-      if (count <= kHertzSort) {
 #pragma unroll
         for (int k = 0; k < kHertzSort; ++k)
           if (k < count)
             take(node[k]);
       } else {
-        for (int last = -1;;) {
+        for (int last = -1, k = 0; k < count; ++k) {
           int best = INT_MAX;
-          for (int q = head; q >= 0; q = H.next[q])
-            if (q > last && q < best)
-              best = q;
-          if (best == INT_MAX)
-            break;
+          for (int q = 0; q < count; ++q) {
+            const int v = mine[q];
+            best = v > last && v < best ? v : best;
+          }
           take(best);
           last = best;
         }
       }
-      H.head[i] = -1;
     }
+    if (many && __syncthreads_or(count > kHertzScan)) {
+      if (tid == 0)
+        sManys = 0;
+      __syncthreads();
+      if (count > kHertzScan)
+        sMany[atomicAdd(&sManys, 1)] = tid;
+      __syncthreads();
+      for (int q = 0; q < sManys; ++q) {
+        const int who = sMany[q], c = H.cnt[base + who], o = H.off[base + who];
+        R* sum = sSum[q & 1];
+        if (tid == who) {
+          sum[0] = f.x, sum[1] = f.y, sum[2] = f.z;
+          sum[3] = t.x, sum[4] = t.y, sum[5] = t.z;
+        }
+        for (int k = tid; k < c; k += kBlock) {
+          const int v = H.slot[o + k];
+          int rank = 0;
+          for (int m = 0; m < c; ++m)
+            rank += H.slot[o + m] < v ? 1 : 0;
+          H.sorted[o + rank] = v;
+        }
+        __syncthreads();
+        R acc = tid < 6 ? sum[tid] : R(0);
+        for (int k0 = 0; k0 < c; k0 += kBlock) {
+          const int m = min(kBlock, c - k0);
+          if (tid < m) {
+            const int node = H.sorted[o + k0 + tid], idx = node >> 1;
+            const V3<R> v = (node & 1) == 0 ? v3(F[idx]) : neg(v3(F[idx]));
+            const V3<R> w = v3((node & 1) == 0 ? TA[idx] : TB[idx]);
+            sVal[0][tid] = v.x, sVal[1][tid] = v.y, sVal[2][tid] = v.z;
+            sVal[3][tid] = w.x, sVal[4][tid] = w.y, sVal[5][tid] = w.z;
+          }
+          __syncthreads();
+          if (tid < 6)
+            for (int j = 0; j < m; ++j)
+              acc = acc + sVal[tid][j];
+          __syncthreads();
+        }
+        if (tid < 6)
+          sum[tid] = acc;
+        __syncthreads();
+        if (tid == who) {
+          f = V3<R>{sum[0], sum[1], sum[2]};
+          t = V3<R>{sum[3], sum[4], sum[5]};
+        }
+      }
+    }
+    if (i >= n)
+      continue;
+    if (count > 0)
+      H.cnt[i] = 0;
     if (candOff)
       for (int q = candOff[i]; q < candOff[i + 1] && q < ncand; ++q)
         if (onW[q]) {
@@ -552,13 +663,23 @@ __global__ void kHertzMaxDisp2(Dev<R> d, int n, const Q4<R>* ref, R* out) {
   blockMaxAtomic(out, mx);  // one atomic per block on the one word
 }
 // carry the shear history onto the rebuilt list (src/sim.hpp:558-585). Both lists are in (first, second
-// body) order, so the old one is searched as it stands; its keys are (larger << 32 | smaller).
+// body) order, so the old one is searched as it stands; its keys are (larger << 32 | smaller). cnt: the
+// pairs of each body.
 __device__ __forceinline__ u64 hertzOrder(u64 k) { return (k << 32) | (k >> 32); }
 template <class R>
 __global__ void kHertzCarry(Dev<R> d, int np, int prevCount, const u64* prevKeys, const Q4<R>* prevXi, u64* keys,
-                            Q4<R>* xi) {
-  GRID_STRIDE(idx, np) {
-    const int2 pr = d.pairs[idx];
+                            Q4<R>* xi, int* cnt) {
+  const int lane = threadIdx.x & 31;
+  for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx - lane < np; idx += (long)gridDim.x * blockDim.x) {
+    const int2 pr = idx < np ? d.pairs[idx] : make_int2(-1, -1);
+    // a body's pairs as the first one are consecutive: one count for the warp's part of them
+    const bool head = __shfl_up_sync(0xffffffffu, pr.x, 1) != pr.x || lane == 0;
+    const unsigned after = __ballot_sync(0xffffffffu, head) >> lane >> 1;
+    if (idx >= np)
+      continue;
+    if (head)
+      atomicAdd(&cnt[pr.x], after ? __ffs(after) : 32 - lane);
+    atomicAdd(&cnt[pr.y], 1);
     const unsigned a = (unsigned)pr.x, b = (unsigned)pr.y;
     const unsigned lo = a < b ? a : b, hi = a < b ? b : a;
     const u64 k = ((u64)hi << 32) | lo, o = hertzOrder(k);

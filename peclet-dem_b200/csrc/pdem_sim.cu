@@ -1285,6 +1285,7 @@ int Sim<R>::findCollisionsVerlet(R margin) {
 }
 template <class R>
 void Sim<R>::detectAll(R margin) {
+  hzRoomValid_ = false;  // the pairs it finds take the Hertz list's place
   const int np = verlet_ ? findCollisionsVerlet(margin) : findCollisionsGrow(margin, posPred_.p);
   mark(ST_NARROW);
   ++launches_, kResetCounters<<<1, 1, 0, stream_>>>(ctr_.p);
@@ -2254,16 +2255,32 @@ void Sim<R>::hertzRebuildPairs(R skin) {
   hzSnPair_.ensure(need, false, stream_);
   hzKeys_.ensure(need, false, stream_);
   hzOn_.ensure(need / 32 + 1, false, stream_);
-  hzNext_.ensure(2 * need, false, stream_);
   cudaCheck(cudaMemsetAsync(hzOn_.p, 0xff, (np / 32 + 1) * sizeof(unsigned), stream_), "memset");
   if (np > 0) {
     ++launches_, kHertzCarry<<<gridFor(np), kBlock, 0, stream_>>>(d_, np, hzPrevCount_, hzPrevKeys_.p, hzPrevXi_.p, hzKeys_.p,
-                                                      hzXi_.p);
+                                                      hzXi_.p, hzCnt_.p);
     KCHECK("hertz carry");
     hzSnPair_.zero(stream_, np);
   }
+  hertzRoom(np);
   hzNumPairs_ = np;
   cudaCheck(cudaMemcpyAsync(hzRefPos_.p, pos_.p, numReal_ * sizeof(Q4<R>), cudaMemcpyDeviceToDevice, stream_), "D2D");
+}
+// the bodies' room for their pairs of the list (HertzTouch), from their counts
+template <class R>
+void Sim<R>::hertzRoom(int np) {
+  const int n = numReal_;
+  // after the offsets: the room taken, and the blocks' flags (HertzTouch::many)
+  const size_t blocks = (size_t)n / kBlock + 1;
+  hzOff_.ensure(n + 1 + (blocks + 3) / 4, false, stream_);
+  hzSlot_.ensure(2 * (size_t)std::max(np, 1), false, stream_);
+  hzSorted_.ensure(2 * (size_t)std::max(np, 1), false, stream_);
+  uint8_t* many = reinterpret_cast<uint8_t*>(hzOff_.p + n + 1);
+  cudaCheck(cudaMemsetAsync(hzOff_.p + n, 0, sizeof(int), stream_), "memset");
+  if (n > 0)
+    ++launches_, kHertzRoom<<<gridFor(n), kBlock, 0, stream_>>>(n, hzCnt_.p, hzOff_.p, hzOff_.p + n, many);
+  KCHECK("hertz room");
+  hzRoomValid_ = true;
 }
 // src/solver_hertz.hpp:343-370
 template <class R>
@@ -2320,8 +2337,13 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
   const R skin = skinFrac * minRad;
   const R rebuildAt = R(0.25) * skin * skin;
   bool rebuild = hzNumPairs_ < 0;
-  hzHead_.ensure(std::max(n, 1), false, stream_);
-  cudaCheck(cudaMemsetAsync(hzHead_.p, 0xff, std::max(n, 1) * sizeof(int), stream_), "memset");
+  hzCnt_.ensure(std::max(n, 1), false, stream_);
+  hzCnt_.zero(stream_, std::max(n, 1));
+  if (!rebuild && !hzRoomValid_) {  // the XPBD step has written the shared list since
+    if (hzNumPairs_ > 0)
+      ++launches_, kHertzCount<<<gridFor(hzNumPairs_), kBlock, 0, stream_>>>(d_, hzNumPairs_, n, hzCnt_.p);
+    hertzRoom(hzNumPairs_);
+  }
   if (!rebuild && hzNumPairs_ > 0)  // the shape may have changed since: every history may be set
     cudaCheck(cudaMemsetAsync(hzOn_.p, 0xff, (hzNumPairs_ / 32 + 1) * sizeof(unsigned), stream_), "memset");
   hzPosRad_.ensure(std::max(capacity_, 1), false, stream_);
@@ -2345,14 +2367,15 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
     qA_.ensure(std::max(np, 1), false, stream_);
     qB_.ensure(std::max(np, 1), false, stream_);
     qC_.ensure(std::max(np, 1), false, stream_);
-    const HertzChains chains{hzHead_.p, hzNext_.p, n};
+    const HertzTouch touch{hzCnt_.p, hzOff_.p, hzSlot_.p, hzSorted_.p,
+                           reinterpret_cast<const uint8_t*>(hzOff_.p + n + 1), n};
     if (np > 0) {
       if (hasShapes)
         ++launches_, kHertzShapePairs<<<gridFor(np), kBlock, 0, stream_>>>(d_, np, P, hzXi_.p, hzSnPair_.p, qA_.p, qB_.p, qC_.p,
-                                                               chains);
+                                                               touch);
       else
         ++launches_, kHertzPairs<<<gridFor(np, kHertzTile), kBlock, 0, stream_>>>(d_, np, P, hzPosRad_.p, hzOn_.p, hzXi_.p, qA_.p,
-                                                                           qB_.p, qC_.p, chains);
+                                                                           qB_.p, qC_.p, touch);
       KCHECK("hertz pairs");
     }
     const int nc = (nw > 0) ? hzNumWallCand_ : 0;
@@ -2367,7 +2390,7 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
     mark(ST_HERTZ_INTEGRATE);
     if (n > 0) {
       ++launches_, kHertzGatherIntegrate<<<gridFor(n), kBlock, 0, stream_>>>(
-          d_, n, chains, qA_.p, qB_.p, qC_.p, nc > 0 ? hzCandOff_.p : nullptr, nc, hzFW_.p, hzTW_.p, hzOnW_.p, g, dt,
+          d_, n, touch, qA_.p, qB_.p, qC_.p, nc > 0 ? hzCandOff_.p : nullptr, nc, hzFW_.p, hzTW_.p, hzOnW_.p, g, dt,
           hasShapes ? 1 : 0, k == 0 ? 1 : 0, hzPosRad_.p);
       KCHECK("hertz integrate");
     }

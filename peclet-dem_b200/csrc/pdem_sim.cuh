@@ -345,7 +345,8 @@ class Sim {
   DBuf<u64> hzKeys_, hzPrevKeys_;
   DBuf<R> hzSnPair_, hzSnWall_;
   DBuf<unsigned> hzOn_;          // pairs whose history may be set, a bit each
-  DBuf<int> hzHead_, hzNext_;    // the bodies' chains of touching pairs
+  DBuf<int> hzCnt_, hzOff_, hzSlot_, hzSorted_;  // the bodies' touching pairs (HertzTouch)
+  bool hzRoomValid_ = false;     // the room is of the pairs that the shared list holds
   DBuf<Q4<R>> hzPosRad_;         // positions with radii
   DBuf<int> hzWallCand_, hzCandOff_, hzOnW_;
   DBuf<Q4<R>> hzFW_, hzTW_;
@@ -543,6 +544,7 @@ class Sim {
   // Hertz engine
   void hertzCommitHistory();
   void hertzRebuildPairs(R skin);
+  void hertzRoom(int np);
   int hertzWallCandidates(R skin);
 };
 

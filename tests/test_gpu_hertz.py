@@ -1,10 +1,12 @@
 """GPU parity of the explicit Hertz-Mindlin engine (`step_hertz`, src/sim.hpp:628-750) through the
 C ABI: tangential history keys and vectors and the state after every call, against the oracle
 restatement (bit-exact at float, within 1e-12 relative at double)."""
+import numpy as np
 import pytest
 
 import parity as P
 import scenes as S
+from peclet.dem import workloads as W
 
 pytestmark = pytest.mark.gpu
 
@@ -106,6 +108,41 @@ def test_failed_rebuild_keeps_the_engine_usable(gpu_api, orc_api, precision, rto
         gpu_api.fn["debug_refuse_alloc"](0)
     assert len(a.debug_hertz()[0]) == 0
     a.step_hertz(2e-6, 16, 0.005)
+    sa, sb = P.snapshot(a, products=False), P.snapshot(b, products=False)
+    (sa["hk"], sa["hx"]), (sb["hk"], sb["hx"]) = a.debug_hertz(), b.debug_hertz()
+    bad = P.diff(sa, sb, rtol=rtol)
+    assert not bad, bad[:4]
+
+
+def _grains(touching, radius=1e-3):
+    """Two large grains, the first and the last body, each covered by `touching` small ones."""
+    k = np.arange(touching) + 0.5
+    phi, theta = np.arccos(1 - 2 * k / touching), np.pi * (1 + 5 ** 0.5) * k
+    u = np.stack([np.cos(theta) * np.sin(phi), np.sin(theta) * np.sin(phi), np.cos(phi)], 1)
+    rho = max(1.5, (touching * 4.6 / (4 * np.pi)) ** 0.5 - 1)
+    reach, r = (rho + 2.1) * radius, np.full(2 * touching + 2, radius)
+    c = np.array([[reach, reach, reach], [3 * reach, reach, reach]])
+    r[0] = r[-1] = rho * radius
+    pos = np.concatenate([c[:1], c[0] + u * (rho + 0.99) * radius, c[1] + u * (rho + 0.99) * radius, c[1:]])
+    im, inertia = W.sphere_props(r, 2500.0)
+    rng = np.random.default_rng(touching)
+    return W.Scene(name="grains", pos=pos, vel=rng.uniform(-0.1, 0.1, pos.shape), inv_mass=im,
+                   inv_inertia=np.repeat(np.asarray(inertia)[:, None], 3, 1), scales=r / radius, global_scale=radius,
+                   domain=((0, 0, 0), (4 * reach, 2 * reach, 2 * reach), (False,) * 3), material=(0.6, 0.0, 0.4),
+                   dt=2e-6)
+
+
+@pytest.mark.parametrize("precision,rtol", [("fp32", 0.0), ("fp64", 1e-12)])
+@pytest.mark.parametrize("touching", [1, 8, 9, 32, 33, 257, 700])
+def test_grains_of_many_contacts(gpu_api, orc_api, touching, precision, rtol):
+    """A body's touching pairs are summed in pair order: in registers, by repeated minimum or by its block,
+    at the edges of each (and of the block's stage of 256)."""
+    sc = _grains(touching)
+    a, b = (P.build(api, sc, lambda s: s.set_hertz_material(0, 1e7, 0.3), precision) for api in (gpu_api, orc_api))
+    for _ in range(2):
+        a.step_hertz(2e-6, 4, 0.3)
+        b.step_hertz(2e-6, 4, 0.3)
+    assert (np.abs(b.debug_hertz()[1]).sum(1) > 0).sum() >= 2 * touching
     sa, sb = P.snapshot(a, products=False), P.snapshot(b, products=False)
     (sa["hk"], sa["hx"]), (sb["hk"], sb["hx"]) = a.debug_hertz(), b.debug_hertz()
     bad = P.diff(sa, sb, rtol=rtol)
