@@ -229,6 +229,31 @@ __global__ void kFlowPack(Dev<R> d, const int* order, const int* coff, int ncol,
     *reinterpret_cast<int4*>(r.rec + t * F::kStride + F::kIds) = make_int4(idx, A, B, f);
   }
 }
+template <class R>
+__device__ __forceinline__ PgsStatic<R> flowRecord(const char* rec, long t, int& idx) {
+  using F = FlowShape<R, 0>;
+  const char* q = rec + t * F::kStride;
+  auto slot = [&](int k) {
+    Q4<R> v;
+    if constexpr (sizeof(R) == 8) {
+      const double2 a = *reinterpret_cast<const double2*>(q + 32 * k), b = *reinterpret_cast<const double2*>(q + 32 * k + 16);
+      v = Q4<R>{a.x, a.y, b.x, b.y};
+    } else {
+      const float4 a = *reinterpret_cast<const float4*>(q + 16 * k);
+      v = Q4<R>{a.x, a.y, a.z, a.w};
+    }
+    return v;
+  };
+  const int4 id = *reinterpret_cast<const int4*>(q + F::kIds);
+  const Q4<R> q0 = slot(0), q1 = slot(1), q2 = slot(2), q3 = slot(3), q4 = slot(4), q5 = slot(5), q6 = slot(6), q7 = slot(7);
+  PgsStatic<R> s;
+  idx = id.x, s.ra = id.y, s.rb = id.z, s.hasB = (id.w & kFlowHasB) != 0;
+  s.Nsq = R(0);  // not read by the update
+  s.N = v3(q0), s.lenN = q0.w, s.TA = v3(q1), s.TB = v3(q2), s.wAn0 = q2.w, s.dc = v3(q3), s.wBn0 = q3.w;
+  s.rAa = v3(q4), s.imA = q4.w, s.rBa = v3(q5), s.imB = q5.w, s.wvN = v3(q6), s.eAvg = q6.w;
+  s.iIA = v3(q7), s.muAvg = q7.w, s.iIB = v3(slot(8)), s.qA = slot(9), s.qB = slot(10);
+  return s;
+}
 // link of each entry's sides to the next entry of the body; targets are mailbox slots of `nb` blocks
 // (block << 14 | slot) or, with nb = 0, entries
 static __global__ void __launch_bounds__(kFlowBlock) kFlowLink(const int* coff, int ncol, const u64* mask, const int* tab,

@@ -75,10 +75,13 @@ __device__ __forceinline__ bool loopBarrier(const GridBar& gb) {
   }
   return gridBarrier(gb);
 }
-// The colour offsets (at most 63 colours) are read once into shared memory.
+// The colour offsets (at most 63 colours) are read once into shared memory. KIND 3: KIND 0 from the
+// per-substep records of kFlowPack (entry t of the order is record t; flowRecord is in pdem_flow.cuh).
+template <class R>
+__device__ __forceinline__ PgsStatic<R> flowRecord(const char* rec, long t, int& idx);
 template <class R, int KIND, int LOOP, bool CLUSTER = false>
 __global__ void __launch_bounds__(kBlock) kSweepLoop(Dev<R> d, const int* order, const int* coff, int ncol, int iters,
-                                                     SolveP<R> P, R thr, GridBar gb) {
+                                                     SolveP<R> P, R thr, GridBar gb, const char* rec) {
   __shared__ int sOff[kSaturatedColor + 2];
   Counters<R>* c = d.ctr;
   volatile int* done = LOOP == 1 ? &c->velDone : LOOP == 2 ? &c->stabDone : &c->posDone;
@@ -104,6 +107,10 @@ __global__ void __launch_bounds__(kBlock) kSweepLoop(Dev<R> d, const int* order,
             pgsOne(d, order[b + t], P, mx, LOOP);
           } else if (KIND == 1) {
             gsOne(d, order[b + t], P, mx);
+          } else if (KIND == 3) {
+            int idx;
+            const PgsStatic<R> st = flowRecord<R>(rec, b + t, idx);
+            pgsCore<R>(d, idx, st, P.eN, P.mu, 0, P, mx);
           } else {
             posGSOne(d, order[b + t], mx);
           }

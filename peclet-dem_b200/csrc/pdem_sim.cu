@@ -323,6 +323,48 @@ bool Sim<R>::launchClusterCfg(K kernel, int blocks, int block, size_t smem, size
   return true;
 }
 
+// this substep's records of the manifolds (KIND 0) or contacts (KIND 2), packed at the first request
+template <class R>
+template <int KIND>
+FlowRecs<R> Sim<R>::flowPack(int ne, int ncol) {
+  using F = FlowShape<R, KIND>;
+  FlowBuf& f = KIND == 0 ? flowM_ : flowC_;
+  if (f.packedAt != substepId_) {
+    f.rec.ensure((size_t)ne * F::kStride, false, stream_);
+    if (KIND == 0)
+      f.var.ensure((size_t)ne, false, stream_);
+    else
+      f.lam.ensure((size_t)ne, false, stream_);
+    f.tab.ensure((size_t)std::max(KIND == 0 ? numReal_ : numParticles_, 1) * ncol, false, stream_);
+  }
+  const FlowRecs<R> rec{f.rec.p, f.var.p, f.lam.p, nullptr, nullptr, 0, 0u};
+  if (f.packedAt != substepId_) {
+    ++launches_, kFlowPack<R, KIND><<<gridFor(ne), kBlock, 0, stream_>>>(
+        d_, KIND == 0 ? mOrder_.p : cOrder_.p, KIND == 0 ? mOff_.p : cOff_.p, ncol, KIND == 0 ? mask_.p : maskP_.p, f.tab.p, rec);
+    KCHECK("flow records");
+    f.packedAt = substepId_;
+    f.blocks = -1;
+  }
+  return rec;
+}
+
+// The velocity loops that flowSweeps leaves, by colour. With a saturated colour, whose serial updates depend
+// on one another, up to sweepClusterEntries_ manifolds run from the packed records in one cluster: a grain
+// with 98 touching neighbours among 10,000 manifolds, FP64, 10 sweeps 2.38 ms (3.31 on the grid), 20 of the
+// stabilization 4.77 (6.68); 32,500 manifolds 2.56 (3.42). Others run on the grid: 25,000 spheres on a floor,
+// one colour, 29 us a substep (39 in a cluster).
+template <class R>
+template <int LOOP>
+void Sim<R>::colourSweeps(int nm, int ncol, int iters, const SolveP<R>& P, R thr) {
+  gbar_.ensure(2, false, stream_);
+  const GridBar gb{gbar_.p, &ctr_.p->err, barrierSleepNs_, barrierSpins_};
+  if (!(ncol > kSaturatedColor && nm <= sweepClusterEntries_ &&
+        launchCluster(kSweepLoop<R, 3, LOOP, true>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncol, iters, P, thr, gb,
+                      (const char*)flowPack<0>(nm, ncol).rec)))
+    launchCoop(kSweepLoop<R, 0, LOOP>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncol, iters, P, thr, gb,
+               (const char*)nullptr);
+}
+
 // One sweep loop as a flow of body states (pdem_flow.cuh) over the manifolds (KIND 0) or contacts
 // (KIND 2) of the substep. Returns false (nothing launched) where the colour order has the saturated
 // colour, which is not an independent set, where no cluster or grid of it can be resident, and for
@@ -342,7 +384,6 @@ bool Sim<R>::flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr) 
   if (ncol > kSaturatedColor || ne >= (1 << 28) || perColor > numSMs_ * kFlowGroup)
     return false;
   FlowBuf& f = KIND == 0 ? flowM_ : flowC_;
-  const int* order = KIND == 0 ? mOrder_.p : cOrder_.p;
   const int* off = KIND == 0 ? mOff_.p : cOff_.p;
   const u64* mask = KIND == 0 ? mask_.p : maskP_.p;
   int nb = 1;
@@ -397,26 +438,12 @@ bool Sim<R>::flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr) 
       return false;
   }
   const int target = cluster ? nb : 0;
-  if (f.packedAt != substepId_ || f.blocks != target) {
-    f.rec.ensure((size_t)ne * F::kStride, false, stream_);
-    if (KIND == 0)
-      f.var.ensure((size_t)ne, false, stream_);
-    else
-      f.lam.ensure((size_t)ne, false, stream_);
-    f.tab.ensure((size_t)std::max(KIND == 0 ? numReal_ : numParticles_, 1) * ncol, false, stream_);
-  }
-  FlowRecs<R> rec{f.rec.p, f.var.p, f.lam.p, nullptr, nullptr, 0, 0u};
-  if (f.packedAt != substepId_) {
-    ++launches_, kFlowPack<R, KIND><<<gridFor(ne), kBlock, 0, stream_>>>(d_, order, off, ncol, mask, f.tab.p, rec);
-    KCHECK("flow records");
-    f.blocks = -1;
-  }
+  FlowRecs<R> rec = flowPack<KIND>(ne, ncol);
   if (f.blocks != target) {
     ++launches_, kFlowLink<<<gridFor(ne, kFlowBlock), kFlowBlock, 0, stream_>>>(
         off, ncol, mask, f.tab.p, KIND == 0 ? mColor_.p : cColor_.p, f.rec.p, F::kStride, F::kIds, target);
     KCHECK("flow links");
   }
-  f.packedAt = substepId_;
   f.blocks = target;
   const GridBar gb{nullptr, &ctr_.p->err, 0u, barrierSpins_};
   ++launches_;
@@ -1746,12 +1773,13 @@ void Sim<R>::demStep() {
       ++launches_, kSweepScenes<R, 1, 1><<<numScenes_, sceneBlock(), 0, s>>>(d_, sceneLpt_.p, mOrder_.p, mOff_.p, velIters_, sp, thr);
     else if (usePGS) {
       if (!flowSweeps<0, 1>(nm, ncolV, velIters_, sp, thr))
-        launchCoop(kSweepLoop<R, 0, 1>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, velIters_, sp, thr, gb);
+        colourSweeps<1>(nm, ncolV, velIters_, sp, thr);
     }
     else if (!usePGS && !(nm <= sweepClusterEntries_ &&
                           launchCluster(kSweepLoop<R, 1, 1, true>, d_, (const int*)mOrder_.p, (const int*)mOff_.p,
-                                        ncolV, velIters_, sp, thr, gb)))
-      launchCoop(kSweepLoop<R, 1, 1>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, velIters_, sp, thr, gb);
+                                        ncolV, velIters_, sp, thr, gb, (const char*)nullptr)))
+      launchCoop(kSweepLoop<R, 1, 1>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, velIters_, sp, thr, gb,
+                 (const char*)nullptr);
     KCHECK("velocity loop");
   }
   // no colours and no fallback: the first sweep is empty, its END finds maxApproach = 0 <= thr
@@ -1845,13 +1873,11 @@ void Sim<R>::demStep() {
       const int iters = stabMode_ == 1 ? 2 * velIters_ : 256;
       const bool stabPersistent = ncolV > 0;
       if (stabPersistent) {
-        gbar_.ensure(2, false, s);
-        const GridBar gb{gbar_.p, &ctr_.p->err, barrierSleepNs_, barrierSpins_};
         ctl(CTL_STAB_BEGIN, R(0), 0);
         if (batch_)
           ++launches_, kSweepScenes<R, 0, 2><<<numScenes_, sceneBlock(), 0, s>>>(d_, sceneLpt_.p, mOrder_.p, mOff_.p, iters, ss, vRestS);
         else if (!flowSweeps<0, 2>(nm, ncolV, iters, ss, vRestS))
-          launchCoop(kSweepLoop<R, 0, 2>, d_, (const int*)mOrder_.p, (const int*)mOff_.p, ncolV, iters, ss, vRestS, gb);
+          colourSweeps<2>(nm, ncolV, iters, ss, vRestS);
       }
       for (int it = 0; it < (stabPersistent ? 0 : iters); ++it) {
         ctl(CTL_STAB_BEGIN, R(0), 0);
@@ -1959,7 +1985,8 @@ void Sim<R>::demStep() {
       tuneEnd();
     }
     else if (!flowSweeps<2, 3>(nc, ncolP, posIters_, sp, posTol))
-      launchCoop(kSweepLoop<R, 2, 3>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP, posIters_, sp, posTol, gb);
+      launchCoop(kSweepLoop<R, 2, 3>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP, posIters_, sp, posTol, gb,
+                 (const char*)nullptr);
     KCHECK("position loop");
   }
   const bool posEmpty = useGS_ && !posDense && ncolP <= 0 && posIters_ > 0 && posTol > R(0);

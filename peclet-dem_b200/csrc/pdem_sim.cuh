@@ -21,6 +21,8 @@
 namespace pdem {
 template <class R>
 struct SolveP;  // pdem_solve.cuh
+template <class R>
+struct FlowRecs;  // pdem_flow.cuh
 
 
 struct CudaError : std::runtime_error {
@@ -435,8 +437,12 @@ class Sim {
   };
   FlowBuf flowM_, flowC_;
   std::map<std::pair<const void*, int>, int> flowOk_;  // residency by (kernel, cluster blocks)
+  template <int KIND>
+  FlowRecs<R> flowPack(int ne, int ncol);
   template <int KIND, int LOOP>
   bool flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr);
+  template <int LOOP>
+  void colourSweeps(int nm, int ncol, int iters, const SolveP<R>& P, R thr);
   void denseSweeps(int nc, int ncol, int left, R tol);
   DBuf<Q4<R>> denseQ_;
   DBuf<int4> denseIds_;

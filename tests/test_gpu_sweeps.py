@@ -65,6 +65,43 @@ def test_flow_own_image(gpu_api, monkeypatch, precision):
     assert a.counters()["manifolds"] > 5
 
 
+def _grain(touching, radius=1e-3):
+    """One large grain, the last body, covered by `touching` small ones that press on it."""
+    k = np.arange(touching) + 0.5
+    phi, theta = np.arccos(1 - 2 * k / touching), np.pi * (1 + 5 ** 0.5) * k
+    u = np.stack([np.cos(theta) * np.sin(phi), np.sin(theta) * np.sin(phi), np.cos(phi)], 1)
+    rho = (touching * 4.6 / (4 * np.pi)) ** 0.5 - 1
+    L = 2 * (rho + 3) * radius
+    pos = np.concatenate([L / 2 + u * (rho + 0.99) * radius, [[L / 2] * 3]])
+    r = np.full(touching + 1, radius)
+    r[-1] = rho * radius
+    im, inertia = W.sphere_props(r, 2500.0)
+    rng = np.random.default_rng(touching)
+    return W.Scene(name="grain", pos=pos, vel=np.concatenate([-0.5 * u, [[0.0] * 3]]) + rng.uniform(-0.1, 0.1, pos.shape),
+                   inv_mass=im, inv_inertia=np.repeat(np.asarray(inertia)[:, None], 3, 1), scales=r / radius,
+                   global_scale=radius, domain=((0, 0, 0), (L, L, L), (False,) * 3),
+                   planes=W.box_planes((0, 0, 0), (L, L, L)), material=(0.5, 0.0, 0.5), dt=1e-5)
+
+
+@pytest.mark.parametrize("precision,rtol", PRECISIONS)
+@pytest.mark.parametrize("entries", [None, 0], ids=["cluster", "grid"])
+@pytest.mark.parametrize("touching,colours", [(62, 62), (63, 63), (200, 63)])
+def test_saturated_manifolds(gpu_api, orc_api, monkeypatch, touching, colours, entries, precision, rtol):
+    """A grain of more touching neighbours than colours: the velocity loops take the saturated colour in
+    manifold order, from the packed records in one cluster or on the grid."""
+    if entries is not None:
+        monkeypatch.setenv("PDEM_SWEEP_CLUSTER_ENTRIES", str(entries))
+    sc = _grain(touching)
+    a, b = P.build(gpu_api, sc, None, precision), P.build(orc_api, sc, None, precision)
+    for k in range(2):
+        a.step(sc.dt)
+        b.step(sc.dt)
+        bad = P.diff(P.snapshot(a), P.snapshot(b), rtol=rtol)
+        assert not bad, f"substep {k}: {bad[:4]}"
+        if k == 0:
+            assert a.counters()["colors_velocity"] == colours
+
+
 @pytest.mark.parametrize("entries", [None, 0], ids=["cluster", "grid"])
 def test_flow_time_out(gpu_api, orc_api, monkeypatch, entries):
     """Every wait of the flow gives up after one poll (a record's copy, a state, the sweep's maximum): no
