@@ -1984,7 +1984,12 @@ void Sim<R>::demStep() {
       ++launches_, kSweepScenes<R, 2, 3><<<numScenes_, sceneBlock(), 0, s>>>(d_, sceneLpt_.p, cOrder_.p, cOff_.p, posIters_, sp, posTol);
       tuneEnd();
     }
-    else if (!flowSweeps<2, 3>(nc, ncolP, posIters_, sp, posTol))
+    // one colour: the first sweep solves every contact, the second finds that and stops, which does not pay for
+    // the flow's records and links (spheres apart on a floor, 50 to 15,000 of them: 14-23 us a substep, 24-34 so)
+    else if (!(ncolP == 1 && nc <= sweepClusterEntries_ &&
+               launchCluster(kSweepLoop<R, 2, 3, true>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP, posIters_,
+                             sp, posTol, gb, (const char*)nullptr)) &&
+             !flowSweeps<2, 3>(nc, ncolP, posIters_, sp, posTol))
       launchCoop(kSweepLoop<R, 2, 3>, d_, (const int*)cOrder_.p, (const int*)cOff_.p, ncolP, posIters_, sp, posTol, gb,
                  (const char*)nullptr);
     KCHECK("position loop");
