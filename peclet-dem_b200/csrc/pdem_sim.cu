@@ -507,7 +507,7 @@ static int bitsFor(long maxValue) {
 
 // The position sweeps of a contact graph with saturated or uncoloured contacts (pdem_dense.cuh). One
 // block while the bodies' positions fit its shared memory and the contacts are few enough for one SM,
-// else the cooperative grid.
+// one cluster up to sweepClusterEntries_ contacts, else the cooperative grid.
 template <class R>
 void Sim<R>::denseSweeps(int nc, int ncol, int left, R tol) {
   cudaStream_t s = stream_;
@@ -518,9 +518,9 @@ void Sim<R>::denseSweeps(int nc, int ncol, int left, R tol) {
   ++launches_, kDensePack<R><<<gridFor(nc), kBlock, 0, s>>>(d_, cOrder_.p, nc, rec);
   KCHECK("dense records");
   const size_t n1 = (size_t)nc + 2;
-  denseRuns_.ensure(5 * n1 + (size_t)nb + 2, false, s);
+  denseRuns_.ensure(6 * n1 + (size_t)nb + 3, false, s);
   int* p = denseRuns_.p;
-  const DenseRuns D{p, p + n1, p + 3 * n1, p + 4 * n1, p + 5 * n1, p + 5 * n1 + nb};
+  const DenseRuns D{p, p + n1, p + 3 * n1, p + 4 * n1, p + 5 * n1, p + 6 * n1, p + 6 * n1 + nb};
   if (ncol > kSaturatedColor) {
     ++launches_, kDenseRuns<R><<<1, 1024, 0, s>>>(d_, cOrder_.p, cOff_.p, nb, D);
     KCHECK("dense runs");
@@ -545,12 +545,14 @@ void Sim<R>::denseSweeps(int nc, int ncol, int left, R tol) {
   ctl(CTL_POS_BEGIN, R(0), 0);
   const size_t smem = (size_t)nb * sizeof(Q4<R>);
   if (smem <= kDenseMaxSmem && nc <= denseOneEntries_) {
-    auto* k = kDenseSweeps<R, true>;
+    auto* k = kDenseSweeps<R, kDenseOne>;
     cudaCheck(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseMaxSmem), "smem attribute");
     ++launches_, k<<<1, kDenseBlock, smem, s>>>(d_, cOff_.p, ncol, posIters_, tol, gb, rec, D, nb, left, inc, qA_.p, iC_.p);
-  } else {
-    launchCoopB(kDenseSweeps<R, false>, kDenseBlock, d_, (const int*)cOff_.p, ncol, posIters_, tol, gb, rec, D, nb, left,
-                inc, qA_.p, iC_.p);
+  } else if (!(nc <= sweepClusterEntries_ &&
+               launchClusterCfg(kDenseSweeps<R, kDenseCluster>, sweepClusterBlocks_, kDenseBlock, 0, 0, d_,
+                                (const int*)cOff_.p, ncol, posIters_, tol, gb, rec, D, nb, left, inc, qA_.p, iC_.p))) {
+    launchCoopB(kDenseSweeps<R, kDenseGrid>, kDenseBlock, d_, (const int*)cOff_.p, ncol, posIters_, tol, gb, rec, D, nb,
+                left, inc, qA_.p, iC_.p);
   }
   KCHECK("dense sweeps");
 }

@@ -160,6 +160,30 @@ def test_dense_forms(gpu_api, orc_api, monkeypatch, n, points, colours, entries,
 
 
 @pytest.mark.parametrize("precision,rtol", PRECISIONS)
+@pytest.mark.parametrize("form", ["block", "cluster", "grid"])
+@pytest.mark.parametrize("scene", ["grain63", "grain64", "grain300", "grains", "stacked120"])
+def test_dense_forms_of_levels(gpu_api, orc_api, monkeypatch, scene, form, precision, rtol):
+    """The saturated contacts in levels of one run (those of one large grain: one warp's outside the one-block
+    form), of a few runs (one block's) and of many: two grains have levels of two runs and then of one, 120
+    cylinders one of 45 and then fewer."""
+    if form != "block":
+        monkeypatch.setenv("PDEM_DENSE_ONE_ENTRIES", "0")
+    if form == "grid":
+        monkeypatch.setenv("PDEM_SWEEP_CLUSTER_ENTRIES", "0")
+    if scene == "grains":
+        sc, b = _grain(75), _grain(110)
+        sc.domain = ((0, 0, 0), tuple(sc.domain[1][k] + b.domain[1][k] for k in range(3)), (False,) * 3)
+        b.pos = b.pos + [float(sc.pos[-1, 0]) * 2, 0, 0]
+        for k in ("pos", "vel", "inv_mass", "inv_inertia", "scales"):
+            setattr(sc, k, np.concatenate([getattr(sc, k), getattr(b, k)]))
+        sc.planes = W.box_planes(*sc.domain[:2])
+    else:
+        sc = _grain(int(scene[5:])) if scene.startswith("grain") else _stacked(120, 512)
+    sim = _compare(gpu_api, orc_api, sc, 2, precision, rtol)
+    assert sim.counters()["colors_position"] == 63
+
+
+@pytest.mark.parametrize("precision,rtol", PRECISIONS)
 @pytest.mark.parametrize("scene", ["bed", "reversed"])
 def test_support_levels_on_the_grid(gpu_api, orc_api, monkeypatch, scene, precision, rtol):
     """The support levels computed by the whole grid (every graph sent there): a bed whose serial sweeps
