@@ -1511,7 +1511,8 @@ void Sim<R>::colorBoth(int nm, int nc, int& ncolV, int& velLeft, int& ncolP, int
     f.sorted.ensure(n2, false, stream_);
     f.state.ensure(n1, false, stream_);
     f.round.ensure(n1, false, stream_);
-    return ColorJob{ne, nb, col, mask, aux, f.cnt.p, f.cnt.p + n1, f.list.p, f.sorted.p, f.state.p, f.round.p};
+    f.item.ensure((size_t)std::max(ne, 1) / 4 + 2, false, stream_);
+    return ColorJob{ne, nb, col, mask, aux, f.cnt.p, f.cnt.p + n1, f.list.p, f.sorted.p, f.state.p, f.round.p, f.item.p};
   };
   const int maxGrid = 4 * numSMs_;
   ColorJob jm = job(neM, nbM, mColor_.p, mask_.p, colorAux_.p, colorM_);
@@ -1535,7 +1536,7 @@ void Sim<R>::colorBoth(int nm, int nc, int& ncolV, int& velLeft, int& ncolP, int
   // stage of a 1,021-sphere bed takes 127 us a substep so, 227 without rounds (each visit crosses L2); a
   // 20,011-sphere bed, whose bodies do not fit, 240 without rounds and 391 with the former grid rounds
   const size_t bodySmem = (size_t)std::max(nbM, nbC) * sizeof(ColorBody);
-  const bool inShared = bodySmem <= kColorMaxSmem && sweepClusterBlocks_ >= 2;
+  const bool inShared = bodySmem <= colorOneBytes_ && sweepClusterBlocks_ >= 2;
   const bool inCluster =
       std::max(neM, neC) <= colorClusterEntries_ && colorBlock_ == kColorBlock &&
       (cudaMemsetAsync(gbar_.p, 0, 2 * sizeof(unsigned), stream_) == cudaSuccess) &&

@@ -238,6 +238,7 @@ class Sim {
     DBuf<int2> sorted;
     DBuf<uint4> state;
     DBuf<u64> round;
+    DBuf<int2> item;
   };
   ColorBuf colorM_, colorC_;
   DBuf<int> sdfState_;
@@ -319,6 +320,11 @@ class Sim {
   long gLog_ = 0, gCheckpoint_ = 0;
   DBuf<int> gscratch_, groundCtl_;
   DBuf<u64> groundT_;
+  // shared memory up to which one block a graph runs the colouring's rounds (PDEM_COLOR_ONE_BYTES)
+  size_t colorOneBytes_ = [] {
+    const char* e = std::getenv("PDEM_COLOR_ONE_BYTES");
+    return e ? (size_t)std::min(std::max(0L, std::strtol(e, nullptr, 10)), 200L * 1024) : (size_t)200 * 1024;
+  }();
   // shared memory up to which one block computes the support levels (PDEM_GROUND_ONE_BYTES)
   size_t groundOneBytes_ = [] {
     const char* e = std::getenv("PDEM_GROUND_ONE_BYTES");

@@ -183,6 +183,20 @@ def test_dense_forms_of_levels(gpu_api, orc_api, monkeypatch, scene, form, preci
     assert sim.counters()["colors_position"] == 63
 
 
+@pytest.mark.parametrize("form", ["shared", "cluster", "grid"])
+@pytest.mark.parametrize("touching", [16, 17, 32, 33, 65, 300])
+def test_colouring_forms(gpu_api, orc_api, monkeypatch, touching, form):
+    """The colouring's rounds in shared memory, its visits without rounds in a cluster and on the grid, with
+    lists sorted by eight lanes (up to 16 entries) or by items of 32: the oracle's colours, on a large grain (a
+    chain as long as its list) and on a bed."""
+    if form == "cluster":
+        monkeypatch.setenv("PDEM_COLOR_ONE_BYTES", "0")
+    if form == "grid":
+        monkeypatch.setenv("PDEM_COLOR_CLUSTER_ENTRIES", "0")
+    _compare(gpu_api, orc_api, _grain(touching), 2, "fp32", 0.0)
+    _compare(gpu_api, orc_api, _bed(20 * touching), 1, "fp32", 0.0)
+
+
 @pytest.mark.parametrize("precision,rtol", PRECISIONS)
 @pytest.mark.parametrize("scene", ["bed", "reversed"])
 def test_support_levels_on_the_grid(gpu_api, orc_api, monkeypatch, scene, precision, rtol):
