@@ -104,7 +104,7 @@ def test_saturated_manifolds(gpu_api, orc_api, monkeypatch, touching, colours, e
 
 @pytest.mark.parametrize("entries", [None, 0], ids=["cluster", "grid"])
 def test_flow_time_out(gpu_api, orc_api, monkeypatch, entries):
-    """Every wait of the flow gives up after one poll (a record's copy, a state, the sweep's maximum): no
+    """Every wait of the flow for another block gives up after one poll (a state, the sweep's maximum): no
     wait is repeated after that, so a loop of 600 sweeps ends at once, the step reports the error, and with
     the default limit the next substeps match the oracle."""
     import time
