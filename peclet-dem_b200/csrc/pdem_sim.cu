@@ -372,9 +372,14 @@ void Sim<R>::colourSweeps(int nm, int ncol, int iters, const SolveP<R>& P, R thr
 // throughput, the records cost more than they save (262,144 periodic spheres, 240,000 contacts: 21.2 ms
 // per ten substeps by colour, 26.3 ms as a flow; 20,011 spheres in a bed, 61,000: 52.7 against 37.4).
 //
+// (Packed beds of 50,000 to 120,000 spheres, which run their full sweeps, would take two thirds of the time as
+// a flow: the line is drawn for the few sweeps of loose packings.)
+//
 // Blocks: one thread-block cluster while its shared memory holds every mailbox (about 14,000 velocity
-// entries in double, 32,768 in float), with about kFlowClusterPer entries of a colour a block, so that a
-// small graph's states travel inside few SMs; else one block a SM or fewer, by kFlowGridPer.
+// entries in double, 32,768 in float; more blocks where those do not hold them: 4,300 manifolds in 43
+// colours, FP64, velocity loop 1,138 us a substep on the grid, 677 so), with about kFlowClusterPer entries of a colour a block, so that a small graph's states travel inside few SMs; else one
+// block a SM or fewer, by kFlowGridPer. With 32 a block a bed of 200 spheres is 5-12 % faster and one of 500 in
+// float 5 % slower, with 128 one of 500 8-12 % slower; from 1,500 spheres all three are equal within 2 %.
 constexpr int kFlowClusterPer = 64, kFlowGridPer = 64;
 template <class R>
 template <int KIND, int LOOP>
@@ -386,11 +391,16 @@ bool Sim<R>::flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr) 
   FlowBuf& f = KIND == 0 ? flowM_ : flowC_;
   const int* off = KIND == 0 ? mOff_.p : cOff_.p;
   const u64* mask = KIND == 0 ? mask_.p : maskP_.p;
+  auto strideOf = [&](int blocks) { return ne / blocks + ncol + 1; };
+  auto smemOf = [&](int blocks) { return F::kStageBytes + (size_t)strideOf(blocks) * F::kSlotBytes; };
+  auto fitsIn = [&](int blocks) {
+    return strideOf(blocks) < (1 << 14) && smemOf(blocks) <= kFlowMaxSmem && ne / (blocks * kFlowGroup) + ncol < kFlowItems;
+  };
   int nb = 1;
-  while (nb < sweepClusterBlocks_ && nb * kFlowClusterPer < perColor)
+  while (nb < sweepClusterBlocks_ && (nb * kFlowClusterPer < perColor || !fitsIn(nb)))
     nb *= 2;
-  const int stride = ne / nb + ncol + 1;
-  const size_t smem = F::kStageBytes + (size_t)stride * F::kSlotBytes;
+  const int stride = strideOf(nb);
+  const size_t smem = smemOf(nb);
   auto* kc = kFlowSweeps<R, KIND, LOOP, true>;
   auto* kg = kFlowSweeps<R, KIND, LOOP, false>;
   cudaLaunchConfig_t cfg{};
@@ -399,8 +409,7 @@ bool Sim<R>::flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr) 
   cfg.stream = stream_;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const bool fits = ne <= sweepClusterEntries_ && stride < (1 << 14) && smem <= kFlowMaxSmem &&
-                    ne / (nb * kFlowGroup) + ncol < kFlowItems;
+  const bool fits = ne <= sweepClusterEntries_ && fitsIn(nb);
   auto resident = [&](const void* k, int blocks) -> int& { return flowOk_.emplace(std::make_pair(k, blocks), -1).first->second; };
   bool cluster = fits;
   if (fits) {

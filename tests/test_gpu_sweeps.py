@@ -102,6 +102,30 @@ def test_saturated_manifolds(gpu_api, orc_api, monkeypatch, touching, colours, e
             assert a.counters()["colors_velocity"] == colours
 
 
+@pytest.mark.parametrize("precision,rtol", PRECISIONS)
+@pytest.mark.parametrize("entries", [None, 0], ids=["cluster", "grid"])
+def test_flow_of_many_colours(gpu_api, orc_api, monkeypatch, entries, precision, rtol):
+    """100 grains of 43 touching neighbours: some 100 entries a colour, whose mailboxes in double need more
+    blocks than the entries of a colour ask for."""
+    if entries is not None:
+        monkeypatch.setenv("PDEM_SWEEP_CLUSTER_ENTRIES", str(entries))
+    one, n = _grain(43), 100
+    L = np.array(one.domain[1])
+    sc = _grain(43)
+    sc.pos = np.concatenate([one.pos + L * [k % 10, k // 10, 0] for k in range(n)])
+    for k in ("vel", "inv_mass", "inv_inertia", "scales"):
+        setattr(sc, k, np.concatenate([getattr(one, k)] * n))
+    sc.domain = ((0, 0, 0), tuple(L * [10, 10, 1]), (False,) * 3)
+    sc.planes = W.box_planes(*sc.domain[:2])
+    a, b = P.build(gpu_api, sc, None, precision), P.build(orc_api, sc, None, precision)
+    a.step(sc.dt)
+    b.step(sc.dt)
+    bad = P.diff(P.snapshot(a), P.snapshot(b), rtol=rtol)
+    assert not bad, bad[:4]
+    c = a.counters()
+    assert c["colors_velocity"] >= 43 and c["manifolds"] >= 4300
+
+
 @pytest.mark.parametrize("entries", [None, 0], ids=["cluster", "grid"])
 def test_flow_time_out(gpu_api, orc_api, monkeypatch, entries):
     """Every wait of the flow for another block gives up after one poll (a state, the sweep's maximum): no
