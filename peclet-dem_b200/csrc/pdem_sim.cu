@@ -376,10 +376,11 @@ void Sim<R>::colourSweeps(int nm, int ncol, int iters, const SolveP<R>& P, R thr
 // a flow: the line is drawn for the few sweeps of loose packings.)
 //
 // Blocks: one thread-block cluster while its shared memory holds every mailbox (about 14,000 velocity
-// entries in double, 32,768 in float; more blocks where those do not hold them: 4,300 manifolds in 43
-// colours, FP64, velocity loop 1,138 us a substep on the grid, 677 so), with about kFlowClusterPer entries of a colour a block, so that a small graph's states travel inside few SMs; else one
-// block a SM or fewer, by kFlowGridPer. With 32 a block a bed of 200 spheres is 5-12 % faster and one of 500 in
-// float 5 % slower, with 128 one of 500 8-12 % slower; from 1,500 spheres all three are equal within 2 %.
+// entries in double, 32,768 in float), with about kFlowClusterPer entries of a colour a block, so that a
+// small graph's states travel inside few SMs, or as many blocks as the mailboxes need (4,300 manifolds in 43
+// colours, FP64, velocity loop 1,138 us a substep on the grid, 677 so); else one block a SM or fewer, by
+// kFlowGridPer. With 32 a block a bed of 200 spheres is 5-12 % faster and one of 500 in float 5 % slower, with
+// 128 one of 500 8-12 % slower; from 1,500 spheres all three are equal within 2 %.
 constexpr int kFlowClusterPer = 64, kFlowGridPer = 64;
 template <class R>
 template <int KIND, int LOOP>
