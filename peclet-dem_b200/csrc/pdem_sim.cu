@@ -464,14 +464,15 @@ bool Sim<R>::flowSweeps(int ne, int ncol, int iters, const SolveP<R>& P, R thr) 
     rec.cap = (long)(f.box.n / (2 * F::kPackets));
     f.ctl.ensure(kFlowCtlWords, false, stream_);
     f.ctl.zero(stream_);
-    if (f.tag > 0xF0000000u) {  // the tags start again
+    const unsigned tags = (unsigned)iters + 2u;
+    if (f.tag > 0xffffffffu - tags) {  // the tags start again
       f.box.zero(stream_);
       f.tag = 0;
     }
     rec.box = f.box.p;
     rec.ctl = f.ctl.p;
     rec.tag0 = f.tag;
-    f.tag += (unsigned)iters + 2u;
+    f.tag += tags;
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.gridDim = dim3(grid);

@@ -65,6 +65,19 @@ def test_flow_own_image(gpu_api, monkeypatch, precision):
     assert a.counters()["manifolds"] > 5
 
 
+def test_flow_tags_start_again(gpu_api, orc_api, monkeypatch):
+    """The mailbox tags of the grid form are numbered through a simulation's launches, as many a launch as it
+    may sweep, and start again when 32 bits are used up: with 0x0f000000 sweeps allowed (of which two spheres
+    on a floor take a few, so that 50 give the same bits) that is within 24 substeps."""
+    monkeypatch.setenv("PDEM_SWEEP_CLUSTER_ENTRIES", "0")
+    a, b = P.build(gpu_api, _bed(2, (10, 0x0F000000)), None, "fp32"), P.build(orc_api, _bed(2, (10, 50)), None, "fp32")
+    for k in range(24):
+        a.step(1e-5)
+        b.step(1e-5)
+        bad = P.diff(P.snapshot(a), P.snapshot(b))
+        assert not bad, f"substep {k}: {bad[:4]}"
+
+
 def _grain(touching, radius=1e-3):
     """One large grain, the last body, covered by `touching` small ones that press on it."""
     k = np.arange(touching) + 0.5
