@@ -1,9 +1,9 @@
-// Persistent loops: the Jones-Plassmann colouring rounds and the coloured Gauss-Seidel sweep loops
-// of the substep, each run as ONE cooperative launch whose blocks are all resident and step
-// through rounds / colours / sweeps together behind a grid-wide barrier. Per-colour and per-round
-// launches (and the host read-back after every colouring round) become barrier crossings of a
-// microsecond or two. The work done per colour, per sweep and per round, and its order, is exactly
-// that of the per-colour kernels (pdem_solve.cuh) and per-round kernels (pdem_contact.cuh).
+// Persistent loops: the two colourings, the coloured Gauss-Seidel sweeps by colour and the support levels,
+// each as ONE launch whose blocks are all resident (a cooperative grid, one thread-block cluster, or a block a
+// scene) and step through phases, colours or sweeps together behind a barrier, where separate launches would
+// need one each and a host read-back. The sweeps' work per colour and its order are those of the per-colour
+// kernels (pdem_solve.cuh); most velocity and position loops run as a flow without colour barriers instead
+// (pdem_flow.cuh).
 #pragma once
 #include "pdem_contact.cuh"
 #include "pdem_solve.cuh"
@@ -65,8 +65,6 @@ __device__ __forceinline__ bool gridBarrier(const GridBar& gb) {
 // (kCtl): each END here is fused with the next sweep's BEGIN. CLUSTER: the launch is one thread-block
 // cluster (a small graph), and the hardware cluster barrier (arrive with release, wait with acquire
 // semantics at cluster scope) replaces the grid-wide one.
-constexpr int kSweepCluster = 8;                                  // blocks of the portable cluster
-constexpr int kSweepClusterEntries = 4 * kSweepCluster * kBlock;  // default largest graph it takes
 template <bool CLUSTER>
 __device__ __forceinline__ bool loopBarrier(const GridBar& gb) {
   if (CLUSTER) {

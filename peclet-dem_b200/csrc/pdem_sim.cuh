@@ -471,9 +471,9 @@ class Sim {
   }();
   long sweepClusterEntries_ = [] {
     const char* e = std::getenv("PDEM_SWEEP_CLUSTER_ENTRIES");
-    // default: up to 8 entries a thread of 16 x 256 (about one entry a thread per colour step at
-    // the 8-12 colours of a settled pile). Measured on the 4,096-sphere settled bed (12.4k
-    // manifolds): the velocity loop 0.57 ms per substep on the cooperative grid, 0.47 in one cluster
+    // Measured on beds, velocity loop of a substep in one cluster and on the grid: 4,700 manifolds 210
+    // and 268 us in FP64, 176 and 212 in FP32; 9,300 222 and 273, 184 and 217; 18,700 280 and 283 (the
+    // mailboxes of the larger ones do not fit in FP64), 203 and 224
     return e ? std::max(0L, std::strtol(e, nullptr, 10)) : 32768L;
   }();
   std::map<std::pair<const void*, int>, int> coopPer_;  // resident blocks per SM, by (kernel, block)

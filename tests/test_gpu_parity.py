@@ -140,11 +140,11 @@ def test_shell_plane_reach_cull(gpu_api, orc_api, precision, rtol):
     _run_pair(gpu_api, orc_api, "shells_at_floor", S.shells_at_floor, None, 4, precision, rtol)
 
 
-@pytest.mark.parametrize("tail", ["0", "4096"])
-def test_colouring_tail_settings(tail):
-    """The colouring's hand-over to one block is a launch-shape setting: with no tail (0) and with
-    the global-memory tail (4096, beyond the shared-memory tables) scenes of every kind stay
-    bit-exact against the oracle (the default, the shared-memory tail, runs in every test above)."""
+@pytest.mark.parametrize("variable", ["PDEM_COLOR_ONE_BYTES", "PDEM_COLOR_CLUSTER_ENTRIES"])
+def test_colouring_form_settings(variable):
+    """The colouring's form is a launch-shape setting: without rounds in a cluster (no shared memory for
+    them) and on the grid (no cluster) scenes of every kind stay bit-exact against the oracle (the default,
+    rounds in shared memory, runs in every test above)."""
     import os
     import subprocess
     import sys
@@ -153,7 +153,7 @@ def test_colouring_tail_settings(tail):
            "or hollow_cylinders or settled_column)")
     r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-m", "gpu", "-k", sel,
                         os.path.join(root, "tests", "test_gpu_parity.py")],
-                       cwd=root, env={**os.environ, "PDEM_COLOR_TAIL": tail}, capture_output=True, text=True)
+                       cwd=root, env={**os.environ, variable: "0"}, capture_output=True, text=True)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     assert "5 passed" in r.stdout, r.stdout[-500:]
 
