@@ -489,27 +489,61 @@ __device__ bool contactLaw(const Model<R>& M, int i, int j, int k, const T* in, 
 //
 // One thread a candidate in blocks of 128: the touching ones (a few percent) need some 100 registers, and
 // small blocks keep more of them resident. Rollout and adjoint over boxes of 2,048 spheres, against blocks of
-// 256: FP64 1.01-1.06 times the speed from 2,048 to 131,072 spheres, FP32 1.01-1.03. (Tiles of 512
-// candidates whose touching ones are listed in shared memory and computed by full warps are equal at 131,072
-// spheres in FP64 and 0.86-0.95 of this speed below 65,536 spheres, both precisions: two block barriers on
-// each block's chain and a quarter of the threads.)
-constexpr int kForwardBlock = 128;
+// 256: FP64 1.01-1.08 times the speed from 2,048 to 131,072 spheres, FP32 1.01-1.03.
+// Long FP64 lists (from kTileFrom candidates) go by tiles: a block tests 512 candidates, four a thread, lists
+// the touching ones in shared memory and computes those with full warps, so that idle lanes do not hold the
+// FP64 pipe. 200 substeps, against one a thread: 98,304 spheres (322,000 candidates) 1.07 times the speed,
+// 131,072 1.03, 65,536 1.02 (over 120 substeps, with fewer contacts, 1.0 at the three); below that, and in FP32,
+// the block barriers and the fewer threads cost more: 0.93 at 2,048 to 16,384 spheres.
+constexpr int kForwardBlock = 128, kTileWays = 4;
+constexpr long kTileFrom = 300000;
+template <class R>
+__device__ __forceinline__ void contactForce(const Model<R>& M, long c, const StateView<R>& s, const StateView<R>& t,
+                                             R* F, R* T) {
+  Contact<R> C;
+  contactPrimal(M, c, s, C);
+  if (!C.active) {
+    st3(t.xi, c, V3<R>{R(0), R(0), R(0)});
+    return;
+  }
+  st3(t.xi, c, C.xi3);
+  atomicAdd3(F, C.i, C.f);
+  atomicAdd3(T, C.i, cross(C.rA, C.f));
+  if (C.j >= 0) {
+    atomicAdd3(F, C.j, mul(C.f, R(-1)));
+    atomicAdd3(T, C.j, cross(C.rB, mul(C.f, R(-1))));
+  }
+}
 template <class R>
 __global__ void __launch_bounds__(kForwardBlock) kContacts(Model<R> M, StateView<R> s, StateView<R> t, R* F, R* T) {
-  GRID_STRIDE(c, M.nc) {
-    Contact<R> C;
-    contactPrimal(M, c, s, C);
-    if (!C.active) {
-      st3(t.xi, c, V3<R>{R(0), R(0), R(0)});
-      continue;
+  GRID_STRIDE(c, M.nc) { contactForce(M, c, s, t, F, T); }
+}
+template <class R>
+__global__ void __launch_bounds__(kForwardBlock) kContactTiles(Model<R> M, StateView<R> s, StateView<R> t, R* F, R* T) {
+  __shared__ int sList[kTileWays * kForwardBlock], sCount;
+  for (long first = (long)blockIdx.x * (kTileWays * kForwardBlock); first < M.nc;
+       first += (long)gridDim.x * (kTileWays * kForwardBlock)) {
+    if (threadIdx.x == 0)
+      sCount = 0;
+    __syncthreads();
+    bool on[kTileWays];
+#pragma unroll
+    for (int q = 0; q < kTileWays; ++q) {
+      const long c = first + q * kForwardBlock + threadIdx.x;
+      on[q] = c < M.nc && contactActive(M, c, s);
     }
-    st3(t.xi, c, C.xi3);
-    atomicAdd3(F, C.i, C.f);
-    atomicAdd3(T, C.i, cross(C.rA, C.f));
-    if (C.j >= 0) {
-      atomicAdd3(F, C.j, mul(C.f, R(-1)));
-      atomicAdd3(T, C.j, cross(C.rB, mul(C.f, R(-1))));
+#pragma unroll
+    for (int q = 0; q < kTileWays; ++q) {
+      const long c = first + q * kForwardBlock + threadIdx.x;
+      if (on[q])
+        sList[atomicAdd(&sCount, 1)] = (int)c;
+      else if (c < M.nc)
+        st3(t.xi, c, V3<R>{R(0), R(0), R(0)});
     }
+    __syncthreads();
+    for (int q = threadIdx.x; q < sCount; q += kForwardBlock)
+      contactForce(M, sList[q], s, t, F, T);
+    __syncthreads();  // the list is read before the next tile's
   }
 }
 // one thread per component (coalesced, three times the threads of one per sphere); the
@@ -1108,7 +1142,9 @@ void forward(const pdem_hz_model* h, int steps, int store, R* traj, R* work, cud
   for (int k = 0; k < steps; ++k) {
     const size_t a = store ? k : (k & 1), b = store ? k + 1 : ((k + 1) & 1);
     const StateView<R> s = view(traj + S * a, M.n), t = view(traj + S * b, M.n);
-    if (M.nc > 0)
+    if (sizeof(R) == 8 && M.nc >= kTileFrom)
+      kContactTiles<R><<<pdem::gridFor(M.nc, kTileWays * kForwardBlock), kForwardBlock, 0, st>>>(M, s, t, F, T);
+    else if (M.nc > 0)
       kContacts<R><<<pdem::gridFor(M.nc, kForwardBlock), kForwardBlock, 0, st>>>(M, s, t, F, T);
     kIntegrate<R><<<pdem::gridFor(3L * M.n), pdem::kBlock, 0, st>>>(M, s, t, F, T);
   }

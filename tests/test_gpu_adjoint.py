@@ -62,6 +62,26 @@ def test_forward_matches_oracle(gpu_api, case, steps):
     assert sim.stats["windows"] == -(-steps // 20)
 
 
+def test_long_candidate_lists_by_tiles(gpu_api):
+    """FP64 lists of 300,000 candidates and more are taken by tiles of 512: the scenes' results are those of
+    the last ones (behind a ragged tile) and the first ones alone, whose short list is taken one a thread."""
+    c = HC.gas(scenes=5000)
+    n = len(c["r"])
+
+    def run(a, b):
+        sim = _sim({**c, **{k: c[k][a:b] for k in ("x0", "v0", "w0", "r", "m", "I")},
+                    "first": list(range(0, b - a + 1, 27))})
+        out, _ = sim.run(*(_t(c[k][a:b], sim) for k in ("x0", "v0", "w0")), HC.THETA, 40)
+        return [o.cpu().numpy() for o in out], sim
+    whole, sim = run(0, n)
+    first = sim.contacts(_t(c["x0"], sim), sim._skin(_t(c["v0"], sim), 20))
+    assert len(first) >= 300000
+    for a, b in ((0, 27 * 15), (n - 27 * 15, n)):
+        part, _ = run(a, b)
+        for x, y, atol in zip(whole, part, (1e-14, 1e-12, 1e-9)):  # force sums are atomics: rounding
+            np.testing.assert_allclose(x[a:b], y, rtol=1e-9, atol=atol)
+
+
 @pytest.mark.parametrize("case,steps", CASES)
 def test_adjoint_matches_dual(gpu_api, case, steps):
     """Adjoint (reverse) and dual (forward) derivatives of the same discrete map: equal to
