@@ -77,7 +77,7 @@ struct HertzP {
 // body of many pairs in order; many: the blocks of kBlock bodies with one that has room for more than
 // kHertzScan. A list that the XPBD step wrote in between may name its ghost slots (n and up): they exert
 // forces, as in the reference, and take none.
-constexpr int kHertzSort = 8, kHertzScan = 32;
+constexpr int kHertzSort = 16, kHertzScan = 32;
 struct HertzTouch {
   int* cnt;
   const int* off;
@@ -90,6 +90,26 @@ __device__ __forceinline__ void hertzNote(const HertzTouch& H, int pair, int i, 
     H.slot[H.off[i] + atomicAdd(&H.cnt[i], 1)] = 2 * pair;
   if (j < H.n)
     H.slot[H.off[j] + atomicAdd(&H.cnt[j], 1)] = 2 * pair + 1;
+}
+// count (at most N) of a body's pairs in ascending order, sorted in registers
+template <int N, class TAKE>
+__device__ __forceinline__ void hertzSorted(const int* mine, int count, TAKE&& take) {
+  int node[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    node[k] = k < count ? mine[k] : INT_MAX;
+#pragma unroll
+  for (int p = 1; p < N; ++p)
+#pragma unroll
+    for (int k = p; k > 0; --k) {
+      const int lo = min(node[k - 1], node[k]), hi = max(node[k - 1], node[k]);
+      node[k - 1] = lo;
+      node[k] = hi;
+    }
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (k < count)
+      take(node[k]);
 }
 // pairs of each body in a list that the XPBD step wrote (a rebuild's kHertzCarry counts its own)
 template <class R>
@@ -150,23 +170,28 @@ __global__ void kHertzPosRad(Dev<R> d, int n, Q4<R>* pr) {
 }
 
 // sphere pairs (src/solver_hertz.hpp:88-144): per-pair force F on i, torques tA on i and tB on j.
-// Some 7 % of the pairs of a packing's Verlet list touch. A block tests a tile, kHertzWays pairs a thread so
-// that their loads are in flight together, then computes the touching ones with full warps. An apart
-// pair's history is cleared only where the pair's bit says that it may be set: on (bit = pair) holds the
-// pairs that touched last, or all after a rebuild. 1.5 million pairs of 262,144 spheres, FP32: 48 us as one
-// thread a pair that cleared every history and wrote a flag for each.
-constexpr int kHertzWays = 4, kHertzTile = kHertzWays * kBlock;
-template <class R>
+// Some 7 % of the pairs of a packing's Verlet list touch. A block tests a tile, WAYS pairs a thread so that
+// their loads are in flight together, then computes the touching ones with full warps. An apart pair's history
+// is cleared only where the pair's bit says that it may be set: on (bit = pair) holds the pairs that touched
+// last, or all after a rebuild. 1.5 million pairs of 262,144 spheres, FP32: 48 us as one thread a pair that
+// cleared every history and wrote a flag for each.
+// WAYS: kHertzWays from kHertzTileFrom pairs, below that one, since the touching pairs of a small list would be
+// few blocks' work in turn. Calls of 100 substeps, four ways against one: 8,000 loose spheres (46,000 pairs) FP64
+// 5.25 and 5.00 ms, 30,000 (174,000) 5.50 and 5.93, 262,144 14.2 and 19.2; FP32 4.96 and 4.61, 5.21 and 5.17, 9.8
+// and 11.5. 8,000 spheres in a close packing, 12 contacts each (60,000): FP64 6.37 and 5.22, FP32 5.28 and 4.50.
+constexpr int kHertzWays = 4, kHertzTileFrom = 100000;
+template <class R, int WAYS>
 __global__ void __launch_bounds__(kBlock) kHertzPairs(Dev<R> d, int np, HertzP<R> P, const Q4<R>* pr, unsigned* on,
                                                       Q4<R>* xi, Q4<R>* F, Q4<R>* TA, Q4<R>* TB, HertzTouch H) {
+  constexpr int kHertzTile = WAYS * kBlock;
   __shared__ int sList[kHertzTile], sCount;
   for (long first = (long)blockIdx.x * kHertzTile; first < np; first += (long)gridDim.x * kHertzTile) {
     if (threadIdx.x == 0)
       sCount = 0;
     __syncthreads();
-    bool touch[kHertzWays];
+    bool touch[WAYS];
 #pragma unroll
-    for (int q = 0; q < kHertzWays; ++q) {
+    for (int q = 0; q < WAYS; ++q) {
       const long idx = first + q * kBlock + threadIdx.x;
       touch[q] = false;
       if (idx < np) {
@@ -181,7 +206,7 @@ __global__ void __launch_bounds__(kBlock) kHertzPairs(Dev<R> d, int np, HertzP<R
       }
     }
 #pragma unroll
-    for (int q = 0; q < kHertzWays; ++q) {
+    for (int q = 0; q < WAYS; ++q) {
       const long idx = first + q * kBlock + threadIdx.x;
       const unsigned now = __ballot_sync(0xffffffffu, touch[q]);
       const long word = idx >> 5;
@@ -489,12 +514,14 @@ __global__ void kHertzWalls(Dev<R> d, int ncand, HertzP<R> P, const int* cand, Q
 // per body: pair contributions in pair order, then wall contributions in wall order; then the
 // symplectic kick-drift (src/solver_hertz.hpp:374-425) with the forces consumed. first: the call's first
 // substep, which takes over what the delta arrays hold (normally zero) and clears them. Up to kHertzSort
-// pairs of a body are sorted in registers, up to kHertzScan taken by repeated minimum; the pairs of a larger
-// grain are ranked by its whole block and summed in that order, one component a thread.
+// pairs of a body are sorted in registers (half of them in a smaller network), up to kHertzScan taken by repeated
+// minimum; the pairs of a larger grain are ranked by its whole block and summed in that order, one component a
+// thread.
 // Before, a thread walked its body's whole incidence list (some 12 pairs, a flag each): 43 us of 262,144
 // spheres, FP32. A call of 40 substeps with one grain of 5 R (147 touching) among 3,000, FP64: 6.3-6.7 ms by
-// that walk, 4.2 so (19.7 by repeated minimum over a chain of all its pairs); eight such among 20,000: 8.3
-// and 5.8.
+// that walk, 4.0 so (19.7 by repeated minimum over a chain of all its pairs); eight such among 20,000: 8.2 and
+// 5.5. 8,000 spheres with 12 contacts each, 100 substeps, FP64: 5.11 ms by the walk, 5.22 so, 5.6 with up to 8
+// sorted in registers.
 template <class R>
 __global__ void __launch_bounds__(kBlock) kHertzGatherIntegrate(Dev<R> d, int n, HertzTouch H, const Q4<R>* F,
                                                                 const Q4<R>* TA, const Q4<R>* TB, const int* candOff,
@@ -528,23 +555,10 @@ __global__ void __launch_bounds__(kBlock) kHertzGatherIntegrate(Dev<R> d, int n,
     const int count = i < n ? H.cnt[i] : 0;
     if (count > 0 && count <= kHertzScan) {
       const int* mine = H.slot + H.off[i];
-      if (count <= kHertzSort) {
-        int node[kHertzSort];
-#pragma unroll
-        for (int k = 0; k < kHertzSort; ++k)
-          node[k] = k < count ? mine[k] : INT_MAX;
-#pragma unroll
-        for (int p = 1; p < kHertzSort; ++p)
-#pragma unroll
-          for (int k = p; k > 0; --k) {
-            const int lo = min(node[k - 1], node[k]), hi = max(node[k - 1], node[k]);
-            node[k - 1] = lo;
-            node[k] = hi;
-          }
-#pragma unroll
-        for (int k = 0; k < kHertzSort; ++k)
-          if (k < count)
-            take(node[k]);
+      if (count <= kHertzSort / 2) {
+        hertzSorted<kHertzSort / 2>(mine, count, take);
+      } else if (count <= kHertzSort) {
+        hertzSorted<kHertzSort>(mine, count, take);
       } else {
         for (int last = -1, k = 0; k < count; ++k) {
           int best = INT_MAX;

@@ -2419,9 +2419,12 @@ void Sim<R>::stepHertz(R dt, int nsteps, R skinFrac) {
       if (hasShapes)
         ++launches_, kHertzShapePairs<<<gridFor(np), kBlock, 0, stream_>>>(d_, np, P, hzXi_.p, hzSnPair_.p, qA_.p, qB_.p, qC_.p,
                                                                touch);
-      else
-        ++launches_, kHertzPairs<<<gridFor(np, kHertzTile), kBlock, 0, stream_>>>(d_, np, P, hzPosRad_.p, hzOn_.p, hzXi_.p, qA_.p,
+      else if (np < kHertzTileFrom)
+        ++launches_, kHertzPairs<R, 1><<<gridFor(np), kBlock, 0, stream_>>>(d_, np, P, hzPosRad_.p, hzOn_.p, hzXi_.p, qA_.p,
                                                                            qB_.p, qC_.p, touch);
+      else
+        ++launches_, kHertzPairs<R, kHertzWays><<<gridFor(np, kHertzWays * kBlock), kBlock, 0, stream_>>>(
+            d_, np, P, hzPosRad_.p, hzOn_.p, hzXi_.p, qA_.p, qB_.p, qC_.p, touch);
       KCHECK("hertz pairs");
     }
     const int nc = (nw > 0) ? hzNumWallCand_ : 0;

@@ -133,7 +133,7 @@ def _grains(touching, radius=1e-3):
 
 
 @pytest.mark.parametrize("precision,rtol", [("fp32", 0.0), ("fp64", 1e-12)])
-@pytest.mark.parametrize("touching", [1, 8, 9, 32, 33, 257, 700])
+@pytest.mark.parametrize("touching", [1, 8, 9, 16, 17, 32, 33, 257, 700])
 def test_grains_of_many_contacts(gpu_api, orc_api, touching, precision, rtol):
     """A body's touching pairs are summed in pair order: in registers, by repeated minimum or by its block,
     at the edges of each (and of the block's stage of 256)."""
@@ -146,6 +146,29 @@ def test_grains_of_many_contacts(gpu_api, orc_api, touching, precision, rtol):
     sa, sb = P.snapshot(a, products=False), P.snapshot(b, products=False)
     (sa["hk"], sa["hx"]), (sb["hk"], sb["hx"]) = a.debug_hertz(), b.debug_hertz()
     bad = P.diff(sa, sb, rtol=rtol)
+    assert not bad, bad[:4]
+
+
+@pytest.mark.parametrize("precision,rtol", [("fp32", 0.0), ("fp64", 1e-12)])
+def test_long_pair_lists(gpu_api, orc_api, precision, rtol):
+    """From 100,000 pairs a thread tests four of a tile: a jittered lattice of 27,000 spheres whose list is above
+    that (the other tests' lists are below), with a ragged last tile."""
+    n, a = 30, 2.02e-3
+    rng = np.random.default_rng(6)
+    g = np.stack(np.meshgrid(*[np.arange(n)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = (g + 0.5) * a + rng.uniform(-3e-5, 3e-5, (n ** 3, 3))
+    im, inertia = W.sphere_props(1e-3, 2500.0)
+    sc = W.Scene(name="lattice", pos=pos, vel=rng.uniform(-0.2, 0.2, pos.shape), inv_mass=np.full(n ** 3, im),
+                 inv_inertia=np.full((n ** 3, 3), inertia), global_scale=1e-3,
+                 domain=((0, 0, 0), (n * a,) * 3, (False,) * 3), material=(0.6, 0.0, 0.4), dt=2e-6)
+    x, y = (P.build(api, sc, lambda s: s.set_hertz_material(0, 1e7, 0.3), precision) for api in (gpu_api, orc_api))
+    for _ in range(2):
+        x.step_hertz(2e-6, 3, 1.0)
+        y.step_hertz(2e-6, 3, 1.0)
+    sx, sy = P.snapshot(x, products=False), P.snapshot(y, products=False)
+    (sx["hk"], sx["hx"]), (sy["hk"], sy["hx"]) = x.debug_hertz(), y.debug_hertz()
+    assert len(sy["hk"]) >= 100000 and len(sy["hk"]) % 1024
+    bad = P.diff(sx, sy, rtol=rtol)
     assert not bad, bad[:4]
 
 
