@@ -58,10 +58,11 @@ constexpr int kBR = 128;   // the reverse kernels (up to 255 registers a thread)
 constexpr int kBPgs = 64;  // the hand-written PGS reverse: one entry a thread, few entries a colour
 // the persistent sweep loops: one cluster of kClusterBlocks blocks (the non-portable size 16),
 // for manifold and contact lists up to kClusterEntries (larger ones sweep colour by colour in separate
-// launches). Measured with the position loops on 2,197 spheres: 53.3 -> 50.1 ms forward + adjoint; the
-// position loops take the line of the PGS loops, their two sides were not timed near it
+// launches, on all SMs). Forward and adjoint of four substeps of a bed, ms in a cluster and by launches:
+// 500 spheres 18.4 and 23.6, 2,197 22.0 and 27.0, 6,000 (18,700 contacts) 26.9 and 29.9, 12,000 (37,300)
+// 37.3 and 31.7, 20,000 48.8 and 34.5
 constexpr int kClusterBlocks = 16;
-constexpr int kClusterEntries = 1 << 16;
+constexpr int kClusterEntries = 24 << 10;
 constexpr int kMaxColours = 62;  // the first saturated colour of the 62-colour masks
 
 __device__ __forceinline__ u64 manKey(int2 ab) {

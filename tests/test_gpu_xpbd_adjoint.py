@@ -127,6 +127,24 @@ def test_hand_reverse_equals_dual_jacobians(gpu_api, monkeypatch):
         np.testing.assert_allclose(a, b, rtol=1e-9, atol=1e-12 * np.abs(b).max())
 
 
+def test_long_lists_by_colour(gpu_api, monkeypatch):
+    """Lists of more than 24,576 entries are swept a launch a colour: the hand-written reverses of a bed of
+    9,261 touching spheres against the reversal through forward-mode local Jacobians, as above."""
+    from peclet.dem import workloads as W
+    sc = W.plain_settling(seed=41, nx=21, ny=21, nz=21, cells_z=24, spacing_r=1.98, jitter_r=0.02, vmax=0.05,
+                          iterations=(4, 4))
+    sc.material = (0.5, 0.3, 0.5)
+    _, g0, t0, _, _ = _gpu(gpu_api, sc, 2)
+    monkeypatch.setenv("PDEM_XADJ_DUAL", "1")
+    _, g1, t1, _, _ = _gpu(gpu_api, sc, 2)
+    np.testing.assert_allclose(t0, t1, rtol=1e-9)
+    for a, b in zip(g0, g1):
+        np.testing.assert_allclose(a, b, rtol=1e-9, atol=1e-12 * np.abs(b).max())
+    sim = P.build(gpu_api, sc, None, "fp64")
+    sim.step(1e-5)
+    assert min(sim.counters()["contacts"], sim.counters()["manifolds"]) > 24576
+
+
 def test_branch_signature_certifies_differences(gpu_api):
     """The record's branch hash is a function of the rollout's branches: the same rollout twice gives
     the same hash; a large change of friction changes it (the cone clamps move)."""
