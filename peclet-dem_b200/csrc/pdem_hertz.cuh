@@ -3,8 +3,8 @@
 // Explicit force model on a cached Verlet pair list: a touching pair's force, torques and Mindlin history
 // are computed by one thread, which notes the pair with its two bodies; each body then takes its
 // pairs' contributions in pair order and its wall contributions in wall order (the reference's atomic
-// order in the serial build), then a symplectic kick-drift. The pair list is rebuilt when any body moved half the skin; the shear
-// history is carried across rebuilds by pair key (sorted keys + binary search).
+// order in the serial build), then a symplectic kick-drift. The pair list is rebuilt when any body moved half
+// the skin; the shear history is carried across rebuilds by pair key (both lists in pair order, binary search).
 #pragma once
 #include <climits>
 

@@ -359,7 +359,8 @@ struct ColorJob {
   int ne, nb;          // entries, bodies
   int* col;            // [ne] colours out
   u64* mask;           // [nb] colours of each body's entries out
-  int* aux;            // [0] list space taken, [1] items of long lists, [2] largest round, [3] max colour, [4] left uncoloured, [5] rounds run
+  int* aux;            // [0] list space taken, [1] items of long lists, [2] largest round, [3] max colour,
+                       // [4] left uncoloured, [5] rounds run
   int *cnt, *at;       // [nb] entries of each body, their place in the lists
   int4* list;          // [2 ne + nb] (key low, key high, entry, other body << 1 | 1 at its first end) unsorted
   int2* sorted;        // [2 ne + nb] (entry, other body (or -1) << 1 | 1 at its first end), then (-1, 0)
@@ -462,8 +463,9 @@ __device__ __forceinline__ void colorFill(const Dev<R>& d, const ColorJob& J, lo
 }
 // each body's list by decreasing key: an element's place is the number of larger keys. Eight lanes a body up
 // to kColorShort entries; longer lists by items of 32 entries, a warp each, with the list's keys passed round
-// by shuffles. The colouring stage of one grain with 3,000, 10,000 and 30,000 contacts: 4.8, 12.9 and 16.8 ms (26.8, 98 and 181
-// by rounds of contention; 69, 550 and 830 with eight lanes a body at any length); of 216 cylinders 0.23 (0.44).
+// by shuffles. The colouring stage of one grain with 3,000, 10,000 and 30,000 contacts: 4.8, 12.9 and 16.8 ms
+// (26.8, 98 and 181 by rounds of contention; 69, 550 and 830 with eight lanes a body at any length); of 216
+// cylinders 0.23 (0.44).
 __device__ __forceinline__ void colorSort(const ColorJob& J, long gtid, long gstride) {
   if (J.ne <= 0)
     return;
